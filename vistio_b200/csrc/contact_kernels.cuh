@@ -503,17 +503,29 @@ __global__ void __launch_bounds__(256) k_al_end(BatchDev B) {
 }
 
 // Per instance: count the pass, record the active contacts, stop or grow mu.
-__global__ void k_al_finish(BatchDev B, uint32_t ninst) {
+// One block: it decides whether the step's loop (handle `again`) runs another
+// pass, which it does while a garment is not done and passes are left. Every
+// garment that is not done has run the same passes.
+constexpr uint32_t kFinishThreads = 512;
+__global__ void __launch_bounds__(kFinishThreads) k_al_finish(BatchDev B, uint32_t ninst, cudaGraphConditionalHandle again,
+                                                              uint32_t max_passes) {
   pdl_begin();
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ninst) return;
   const StepParams& P = *B.prm;
-  InstRed& R = B.red[k];
-  if (R.al_done) return;
-  R.al_iters += 1;
-  R.last_active = R.active;
-  if (__uint_as_float(R.maxviol_bits) < P.al_tolerance) R.al_done = 1;
-  else R.mu *= P.al_mu_growth;
+  bool more = false;
+  for (uint32_t k = threadIdx.x; k < ninst; k += kFinishThreads) {
+    InstRed& R = B.red[k];
+    if (R.al_done) continue;
+    R.al_iters += 1;
+    R.last_active = R.active;
+    if (__uint_as_float(R.maxviol_bits) < P.al_tolerance) {
+      R.al_done = 1;
+    } else {
+      R.mu *= P.al_mu_growth;
+      more = more || R.al_iters < max_passes;
+    }
+  }
+  more = __syncthreads_or(more);
+  if (threadIdx.x == 0) cudaGraphSetConditional(again, more ? 1u : 0u);
 }
 
 // Zeroes the FP64 self-contact gradient accumulator before a detect.
