@@ -969,6 +969,7 @@ vistio_status capture(vistio_batch* b, bool ipc, bool self, cudaGraphExec_t* out
     launch_pdl(k_finalize, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
   } else {
     if (b->cfg.al_max_iterations) {
+      if (self) L += launch_self_sort(b->dev, b->self.view(), b->n_tri_chunks, st);
       cudaStreamCaptureStatus status;
       const cudaGraphNode_t* deps = nullptr;
       size_t ndeps = 0;
@@ -1986,6 +1987,7 @@ vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const ui
     return e == cudaErrorMemoryAllocation ? VISTIO_ERR_OOM : VISTIO_ERR_GPU;
   };
   uint32_t n = uint32_t(tris.size());
+  S.tall = 0;
   std::vector<SelfInst> si(n);
   std::vector<uint32_t> tri_inst(T);
   uint64_t tb = 0, boxes = 0;
@@ -2007,6 +2009,7 @@ vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const ui
       cnt = (cnt + 1) / 2;
     }
     I.nlevels = l;
+    S.tall = S.tall || l > kLeafLevels + 1;
     boxes += off;
     for (uint32_t t = 0; t < nt; ++t) tri_inst[tb + t] = k;
     tb += nt;
@@ -2066,6 +2069,7 @@ vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const ui
     SA(S.order_alt, Tn * 4);
     SA(S.sort_hist, 256ull * S.sort_blocks * 4);
     SA(S.sort_sums, (S.sort_scan_blocks + 1ull) * 4);
+    SA(S.bounds, 24ull * n);
     S.leaf_tri = S.sort_passes % 2 == 0 ? S.order : S.order_alt;  // where the last pass leaves the order
   }
   // the self CCD's deduplicated tests: as many as the pair capacity (a cloth
@@ -2131,8 +2135,8 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
   std::vector<uint32_t> nvs{nv}, vb{0};
   vistio_status r = self_build(S, tl, nvs, vb, nt, st, err);
   if (r != VISTIO_OK) return r;
-  launch_self_sort(d, S.view(), st);
-  k_self_boxes<<<1, 1024, 0, st>>>(d, S.view(), margin);
+  launch_self_sort(d, S.view(), uint32_t(ch.size()), st);
+  launch_self_boxes(d, S.view(), uint32_t(ch.size()), margin, st);
   k_self_count<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
   k_scan_local<<<S.scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
   k_scan_sums<<<1, kScanBlock, 0, st>>>(S.block_sums, S.scan_blocks, S.npairs);
@@ -2394,7 +2398,8 @@ vistio_status broadphase_pairs_noalloc_impl(vistio_ctx* ctx, uint32_t nv, const 
                                          reinterpret_cast<const uint32_t*>(at(NaLayout::raw_tri)), nt,
                                          d.pos, reinterpret_cast<uint4*>(at(NaLayout::tri)), S.tri_inst,
                                          reinterpret_cast<int4*>(at(NaLayout::chunks)), nchunks);
-  k_self_boxes<<<1, 1024, 0, st>>>(d, S, margin);
+  S.tall = I.nlevels > kLeafLevels + 1;
+  launch_self_boxes(d, S, nchunks, margin, st);
   k_self_count<<<nchunks, kElemThreads, 0, st>>>(d, S);
   k_scan_local<<<scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
   k_scan_sums<<<1, kScanBlock, 0, st>>>(S.block_sums, scan_blocks, S.npairs);
