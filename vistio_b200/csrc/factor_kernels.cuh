@@ -103,9 +103,16 @@ __global__ void __launch_bounds__(kPivotRows) k_fpivot(FrontDev D, const uint2* 
   const double* F = D.fronts + D.front_off[it.x];
   double* V = D.work + D.work_off[it.x];
   double* Q = V + uint64_t(nf) * kPivots;
-  for (uint32_t e = tid; e < b * b; e += kPivotRows) {
-    const uint32_t i = e / b, j = e % b;
-    P[i][j] = F[uint64_t(k0 + max(i, j)) * nf + k0 + min(i, j)];
+  // the block, padded to 32 pivots by the identity: thread tid holds column
+  // tid & 31 of the rows tid / 32 + 4 u
+  constexpr uint32_t kRows = kPivots * kPivots / kPivotRows;
+  const uint32_t pj = tid & 31, pi = tid >> 5;
+  double x[kRows];
+#pragma unroll
+  for (uint32_t u = 0; u < kRows; ++u) {
+    const uint32_t i = pi + 4 * u;
+    x[u] = i < b && pj < b ? F[uint64_t(k0 + max(i, pj)) * nf + k0 + min(i, pj)] : i == pj ? 1.0 : 0.0;
+    P[i][pj] = x[u];
   }
   __syncthreads();
   // in-place inverse by Gauss-Jordan steps; the pivots are those of a Cholesky
@@ -116,49 +123,42 @@ __global__ void __launch_bounds__(kPivotRows) k_fpivot(FrontDev D, const uint2* 
       bad = true;
       d = 1.0;  // keep going with finite numbers; the host reports the failure
     }
-    const double inv = 1.0 / d;
-    double nv[kPivots * kPivots / kPivotRows];
-    uint32_t n = 0;
+    const double inv = 1.0 / d, row = P[k][pj] * inv;
 #pragma unroll
-    for (uint32_t e0 = 0; e0 < kPivots * kPivots; e0 += kPivotRows, ++n) {
-      const uint32_t e = e0 + tid;
-      if (e >= b * b) continue;
-      const uint32_t i = e / b, j = e % b;
-      const double col = P[i][k], row = P[k][j];
-      nv[n] = i == k ? (j == k ? inv : row * inv) : j == k ? -col * inv : P[i][j] - col * row * inv;
+    for (uint32_t u = 0; u < kRows; ++u) {
+      const uint32_t i = pi + 4 * u;
+      const double col = P[i][k];
+      x[u] = i == k ? (pj == k ? inv : row) : pj == k ? -col * inv : x[u] - col * row;
     }
     __syncthreads();
-    n = 0;
 #pragma unroll
-    for (uint32_t e0 = 0; e0 < kPivots * kPivots; e0 += kPivotRows, ++n) {
-      const uint32_t e = e0 + tid;
-      if (e < b * b) P[e / b][e % b] = nv[n];
-    }
+    for (uint32_t u = 0; u < kRows; ++u) P[pi + 4 * u][pj] = x[u];
     __syncthreads();
   }
   if (bad && tid == 0) atomicOr(D.status, 32u);
   if (it.y == 0) {
     double* Pw = Q + uint64_t(nf) * kPivots;
-    for (uint32_t e = tid; e < b * b; e += kPivotRows) Pw[(e / b) * kPivots + e % b] = P[e / b][e % b];
+    for (uint32_t e = tid; e < kPivots * kPivots; e += kPivotRows) Pw[e] = P[e / kPivots][e % kPivots];
   }
   const uint32_t i = it.y * kPivotRows + tid;
   if (i >= nf || (i >= k0 && i < k0 + b)) return;
-  // V_i: right of the diagonal block its row, left of it (already eliminated)
-  // minus its column of the pivot rows
+  // V_i: below the block its row, before it (already eliminated) minus its
+  // column of the pivot rows
   double w[kPivots];
 #pragma unroll
   for (uint32_t q = 0; q < kPivots; ++q)
     w[q] = q >= b ? 0.0 : i > k0 ? F[uint64_t(i) * nf + k0 + q] : -F[uint64_t(k0 + q) * nf + i];
 #pragma unroll
   for (uint32_t q = 0; q < kPivots; ++q) V[uint64_t(i) * kPivots + q] = w[q];
+#pragma unroll 4
   for (uint32_t j = 0; j < kPivots; ++j) {
-    double a = 0.0;
-    if (j < b) {
+    double a0 = 0.0, a1 = 0.0;
 #pragma unroll
-      for (uint32_t q = 0; q < kPivots; ++q)
-        if (q < b) a += w[q] * P[q][j];
+    for (uint32_t q = 0; q < kPivots; q += 2) {
+      a0 += w[q] * P[q][j];
+      a1 += w[q + 1] * P[q + 1][j];
     }
-    Q[uint64_t(i) * kPivots + j] = a;
+    Q[uint64_t(i) * kPivots + j] = a0 + a1;
   }
 }
 
