@@ -207,9 +207,8 @@ __global__ void __launch_bounds__(256) k_detect(BatchDev B, int mode) {
 // CCD step bound for the colliders (ground_plane.rs:112-134, sphere.rs:178-224,
 // cylinder.rs:201-262, box_collider.rs:203-251)
 // and the backtracking sum grad . d over free vertices (pd_solver.rs:915-925).
-__global__ void __launch_bounds__(256) k_ccd(BatchDev B) {
-  pdl_begin();
-  int4 ch = B.vtx_chunks[blockIdx.x];
+__device__ __forceinline__ void collider_ccd(const BatchDev& B, uint32_t chunk) {
+  int4 ch = B.vtx_chunks[chunk];
   const StepParams& P = *B.prm;
   InstRed& R = B.red[ch.x];
   if (R.al_done) return;
@@ -298,6 +297,11 @@ __global__ void __launch_bounds__(256) k_ccd(BatchDev B) {
     if (toi < 1.f) atomicMin(&R.toi_bits, __float_as_uint(fmaxf(toi, 0.f)));
     if (gdd != 0.0) atomicAdd(&R.gdd, gdd);
   }
+}
+
+__global__ void __launch_bounds__(256) k_ccd(BatchDev B) {
+  pdl_begin();
+  collider_ccd(B, blockIdx.x);
 }
 
 // The colliders of the runner's non-IPC path (runner.rs:212-218 then

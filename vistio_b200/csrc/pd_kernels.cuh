@@ -449,9 +449,41 @@ __global__ void __launch_bounds__(128, 8) k_hinge2(BatchDev B) {
   if (two) B.hinge_out[h1] = hinge_project(sb, wb, b0, b1, b2, b3);
 }
 
+// Both local steps of a small batch in one launch: blocks [0, ntri) one chunk
+// of triangles, the rest one chunk of hinges, one element per thread. A small
+// batch's iteration is a chain of launches of 2 to 3 us each, whatever they do
+// (sheet 20x20: 10 launches, 29 us); large ones keep a kernel each, in the
+// shapes the autotuner times.
+__global__ void __launch_bounds__(256, 4) k_local(BatchDev B, uint32_t ntri) {
+  pdl_begin();
+  const bool tri = blockIdx.x < ntri;
+  const int4 ch = tri ? B.tri_chunks[blockIdx.x] : B.hinge_chunks[blockIdx.x - ntri];
+  if ((int)threadIdx.x >= ch.z) return;
+  if (B.prm->ipc && B.red[ch.x].al_done) return;
+  const uint32_t e = uint32_t(ch.y) + threadIdx.x;
+  if (tri) {
+    const InstDev I = B.inst[ch.x];
+    const uint4 a = B.tri_idx[e];
+    tri_project(B, I, e, B.tri_dm[e], B.tri_w[e], B.pos[a.x], B.pos[a.y], B.pos[a.z]);
+  } else {
+    const uint4 id = B.hinge_idx[e];
+    const float4 st = B.inst[ch.x].unit_stencils ? make_float4(-1.f, -1.f, 1.f, 1.f) : B.hinge_st[e];
+    B.hinge_out[e] = hinge_project(st, B.hinge_wr[e], f3(B.pos[id.x]), f3(B.pos[id.y]), f3(B.pos[id.z]), f3(B.pos[id.w]));
+  }
+}
+
+__device__ __forceinline__ void red_reset(InstRed& R) {
+  R.diff_sq = 0.0;
+  R.norm_sq = 0.0;
+  R.toi_bits = __float_as_uint(1.0f);
+  R.gdd = 0.0;
+}
+
 // Residual gather: r_i = m_i (pred_i / dt^2 - x_i / h^2) + sum of element
 // terms [- (mu grad_i + lambda_i)], written in solve (permuted) order.
-// keep_rhs also stores r in R0 for a refinement of this iteration's solve.
+// keep_rhs also stores r in R0 for a refinement of this iteration's solve. A
+// garment's first block counts the iteration and clears the sums of its solve
+// (their readers in the last iteration are done).
 __global__ void __launch_bounds__(256) k_gather(BatchDev B, int keep_rhs) {
   pdl_begin();
   int4 ch = B.vtx_chunks[blockIdx.x];
@@ -461,6 +493,10 @@ __global__ void __launch_bounds__(256) k_gather(BatchDev B, int keep_rhs) {
   const StepParams& P = *B.prm;
   InstRed& R = B.red[ch.x];
   if (P.ipc && R.al_done) return;
+  if (g == I.vbase) {
+    red_reset(R);
+    R.iters += 1;
+  }
   float m = B.mass[g];
   float3 x = f3(B.pos[g]), q = f3(B.pred[g]);
   float cm = m * I.inv_hmat2, cr = m * P.inv_dt2;
@@ -511,17 +547,14 @@ __device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
   return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, 0.f);
 }
 
-// Clears the per-instance residual sums before a solve.
+// Clears the per-instance residual sums before a solve of its own (without a gather).
 __global__ void k_red_reset(BatchDev B, uint32_t ninst) {
   pdl_begin();
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ninst) return;
   InstRed& R = B.red[k];
   if (B.prm->ipc && R.al_done) return;
-  R.diff_sq = 0.0;
-  R.norm_sq = 0.0;
-  R.toi_bits = __float_as_uint(1.0f);
-  R.gdd = 0.0;
+  red_reset(R);
 }
 
 // Iterative refinement of the global solve: T = R0 - A d in FP64, with d the
@@ -609,7 +642,6 @@ __global__ void __launch_bounds__(128) k_update(BatchDev B, int do_update, int a
     atomicAdd(&R.diff_sq, dsq);
     atomicAdd(&R.norm_sq, nsq);
   }
-  if (threadIdx.x == 0 && ch.y == int(I.vbase)) R.iters += 1;
 }
 
 // Whole-batch positions between interleaved xyz (the host layout, one
