@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <iterator>
 #include <limits>
 #include <condition_variable>
 #include <memory>
@@ -530,8 +531,8 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
   // Merge the supernodal tree into few levels. A sweep's time on a small batch
   // is the number of dependent levels, not the factor's bytes: each level costs
   // a signal and a few round trips through L2 whatever its size. So every
-  // subtree of at most kMergeCols[0] columns becomes one supernode, then every
-  // subtree of what remains of at most kMergeCols[1] columns, and so on; the
+  // subtree of at most the first of kMergeCols' limits becomes one supernode,
+  // then every subtree of what remains of at most the second, and so on; the
   // last limit repeats until nothing remains. Rows below a merged supernode are
   // those of its topmost part (the parts below it only reach into the merged
   // columns and those rows).
@@ -541,8 +542,10 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
     for (uint32_t j = sns[k].f; j < sns[k].f + sns[k].s; ++j) fine_of[j] = k;
   for (uint32_t k = 0; k < nfine; ++k)
     if (!sns[k].below.empty()) fine_parent[k] = fine_of[sns[k].below[0]];
+  const MergeCols* merge = kMergeCols;
+  while (n > merge->max_n) ++merge;
   for (uint32_t l = 0, left = nfine; left; ++l) {
-    const uint64_t limit = kMergeCols[std::min<uint32_t>(l, kMergeLevels - 1)];
+    const uint64_t limit = merge->cols[std::min<size_t>(l, std::size(merge->cols) - 1)];
     std::vector<uint64_t> cols(nfine, 0);
     for (uint32_t k = 0; k < nfine; ++k) {  // children precede parents
       if (head[k] != UINT32_MAX) continue;

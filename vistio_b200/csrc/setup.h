@@ -30,11 +30,25 @@ struct SetupParams {
 
 // Largest fundamental supernode (columns) before the tree is merged.
 constexpr uint32_t kMaxSupernodeCols = 256;
-// The supernodal tree is merged into few levels: subtrees of at most
-// kMergeCols[0] columns become one supernode each, then subtrees of the rest
-// of at most kMergeCols[1] columns, and so on (the last limit repeats).
-constexpr uint32_t kMergeLevels = 5;
-constexpr uint32_t kMergeCols[kMergeLevels] = {32, 96, 288, 864, 1024};
+// The supernodal tree is merged into few levels: subtrees of at most cols[0]
+// columns become one supernode each, then subtrees of the rest of at most
+// cols[1] columns, and so on (the last limit repeats). Wide limits give fewer
+// levels, which bound a few garments, and more factor bytes, which bound many.
+// The garment's size alone decides (its result must not depend on its batch);
+// plain steps of 10 iterations (us, one garment / 16 / 128 of it) with the three
+// rows below, the one taken marked:
+//   side  45    *211 /  332 / 1421    266 /  341 / 1394    322 /  399 / 1420
+//         64    *271 /  541 / 2618    280 /  554 / 2619    348 /  519 / 2491
+//         97     292 / 1070 / 5893   *332 / 1078 / 5546    401 / 1096 / 5374
+//        121     346 / 1821 / 10721   356 / 1613 / 8844   *414 / 1600 / 8094
+//        150     420 / 2604 / 15820   412 / 2504 / 14505  *443 / 2353 / 12526
+struct MergeCols {
+  uint32_t max_n;    // vertices up to which the row is taken
+  uint32_t cols[5];
+};
+constexpr MergeCols kMergeCols[] = {{5000, {128, 512, 1024, 1024, 1024}},
+                                    {11000, {48, 160, 512, 1024, 1024}},
+                                    {0xffffffffu, {32, 80, 200, 500, 1024}}};
 constexpr uint32_t kBottomLevel = 0xffffffffu;  // level of a leaf of the merged tree
 // Floats of one supernode's two panels as packed for the GPU (see SnDev):
 // forward, s columns of m + s rows; backward, m columns of s rows; rows padded
