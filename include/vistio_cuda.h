@@ -480,15 +480,14 @@ vistio_status vistio_sparse_destroy(vistio_factor* f);
 
 /* ---- contact boundary queries ---- */
 /* Candidate triangle pairs (ta < tb) whose AABBs inflated by `margin` overlap,
- * computed on the GPU (balanced tree over mesh-order triangles, count / scan /
- * write). Writes up to `cap` pairs sorted; *count = total. */
+ * computed and sorted on the GPU. Writes up to `cap` pairs sorted; *count = total. */
 vistio_status vistio_broadphase_pairs(vistio_ctx* ctx, uint32_t nv, const float* px, const float* py, const float* pz,
                                       uint32_t nt, const uint32_t* tris, float margin, uint32_t* pairs, uint64_t cap,
                                       uint64_t* count);
 /* Allocation-free variant of vistio_broadphase_pairs (no counterpart in the
  * reference). Same inputs and the same sorted pair list, but the call allocates
  * and frees no device memory: every buffer it uses lives in one fixed region
- * (about 16 MB) built into the library. For callers that cannot allocate on
+ * (about 20 MB) built into the library. For callers that cannot allocate on
  * the call: a server whose device memory is fully committed to resident
  * garments (a cudaMalloc could fail there), or a per-frame collision query on
  * a latency-critical thread, where cudaFree would synchronise the whole device.

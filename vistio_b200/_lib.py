@@ -11,6 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libvistio_b200.so")
 
 OK = 0
+CAPACITY = 12
 STATUS_NAMES = {
     0: "OK", 1: "INVALID_MESH", 2: "INVALID_MATERIAL", 3: "INVALID_CONFIG", 4: "IO", 5: "SERIALIZATION",
     6: "GPU", 7: "SOLVER_DIVERGENCE", 8: "INVARIANT", 9: "TIMEOUT", 10: "OOM", 11: "NOT_SPD", 12: "CAPACITY",

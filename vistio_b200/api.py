@@ -591,12 +591,17 @@ def broadphase_pairs(pos: np.ndarray, tris: np.ndarray, margin: float, ctx: Opti
     cols = [np.ascontiguousarray(pos[:, k]) for k in range(3)]
     cnt = C.c_uint64()
     u32 = C.POINTER(C.c_uint32)
-    L.check(L.lib().vistio_broadphase_pairs(ctx.h, pos.shape[0], *[_fp(c) for c in cols], tris.shape[0],
-                                            tris.ctypes.data_as(u32), float(margin), None, 0, C.byref(cnt)), ctx.h)
-    out = np.zeros((max(cnt.value, 1), 2), np.uint32)
-    L.check(L.lib().vistio_broadphase_pairs(ctx.h, pos.shape[0], *[_fp(c) for c in cols], tris.shape[0],
-                                            tris.ctypes.data_as(u32), float(margin), out.ctypes.data_as(u32),
-                                            cnt.value, C.byref(cnt)), ctx.h)
+    # one call into room for the usual number of pairs; a second if there are more
+    room = 32 * tris.shape[0] + 64
+    while True:
+        out = np.empty((room, 2), np.uint32)
+        status = L.lib().vistio_broadphase_pairs(ctx.h, pos.shape[0], *[_fp(c) for c in cols], tris.shape[0],
+                                                 tris.ctypes.data_as(u32), float(margin), out.ctypes.data_as(u32), room,
+                                                 C.byref(cnt))
+        if status != L.CAPACITY or cnt.value <= room:
+            break
+        room = cnt.value
+    L.check(status, ctx.h)
     return out[: cnt.value]
 
 

@@ -1990,10 +1990,12 @@ vistio_status vistio_barrier_grad(vistio_ctx* ctx, uint32_t n, const double* d2,
 namespace vistio {
 
 namespace {
-// Builds the per-garment tree layout and the exclusion lists.
+// Builds the per-garment tree layout and, for the steps of a batch, the
+// exclusion lists and the self CCD's test list (the broad-phase entry points
+// use neither).
 vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const uint32_t*, uint32_t>>& tris,
                          const std::vector<uint32_t>& nverts, const std::vector<uint32_t>& vbase, uint64_t T,
-                         cudaStream_t st, std::string* err) {
+                         bool step, cudaStream_t st, std::string* err) {
   auto bad = [&](cudaError_t e, const char* what) {
     if (err) *err = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? VISTIO_ERR_OOM : VISTIO_ERR_GPU;
@@ -2029,8 +2031,9 @@ vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const ui
   // exclusion lists: 1-ring plus the vertex (exclusion.rs:27-58, depth 1), global ids
   uint64_t V = 0;
   for (uint32_t k = 0; k < n; ++k) V = std::max<uint64_t>(V, uint64_t(vbase[k]) + nverts[k]);
+  if (!step) V = 0;
   std::vector<std::vector<uint32_t>> ring(V);
-  for (uint32_t k = 0; k < n; ++k) {
+  for (uint32_t k = 0; k < n && step; ++k) {
     const uint32_t* t = tris[k].first;
     for (uint32_t i = 0; i < tris[k].second; ++i) {
       uint32_t v[3] = {vbase[k] + t[3 * i], vbase[k] + t[3 * i + 1], vbase[k] + t[3 * i + 2]};
@@ -2086,18 +2089,20 @@ vistio_status self_build(SelfContactDev& S, const std::vector<std::pair<const ui
   }
   // the self CCD's deduplicated tests: as many as the pair capacity (a cloth
   // mesh has about 1.6 per pair); beyond it the CCD runs over the pairs
-  S.vt_cap = std::min<uint64_t>(S.pair_cap, 0xffffffffull);
-  SA(S.leaf_of, std::max<uint64_t>(T, 1) * 4);
-  SA(S.vt, S.vt_cap * sizeof(uint2));
-  SA(S.nvt, 8);
+  if (step) {
+    S.vt_cap = std::min<uint64_t>(S.pair_cap, 0xffffffffull);
+    SA(S.leaf_of, std::max<uint64_t>(T, 1) * 4);
+    SA(S.vt, S.vt_cap * sizeof(uint2));
+    SA(S.nvt, 8);
+  }
 #undef SA
   if ((e = cudaMemcpyAsync(S.inst, si.data(), n * sizeof(SelfInst), cudaMemcpyHostToDevice, st)) != cudaSuccess) return bad(e, "copy");
   if (T && (e = cudaMemcpyAsync(S.tri_inst, tri_inst.data(), T * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) return bad(e, "copy");
   if ((e = cudaMemcpyAsync(S.adj_ptr, aptr.data(), (V + 1) * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) return bad(e, "copy");
   if (!adj.empty() && (e = cudaMemcpyAsync(S.adj, adj.data(), adj.size() * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) return bad(e, "copy");
   if ((e = cudaMemsetAsync(S.npairs, 0, 8, st)) != cudaSuccess) return bad(e, "memset");
-  if ((e = cudaMemsetAsync(S.nvt, 0, 8, st)) != cudaSuccess) return bad(e, "memset");
-  if ((e = cudaMemsetAsync(S.leaf_of, 0, std::max<uint64_t>(T, 1) * 4, st)) != cudaSuccess) return bad(e, "memset");
+  if (step && (e = cudaMemsetAsync(S.nvt, 0, 8, st)) != cudaSuccess) return bad(e, "memset");
+  if (step && (e = cudaMemsetAsync(S.leaf_of, 0, std::max<uint64_t>(T, 1) * 4, st)) != cudaSuccess) return bad(e, "memset");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return bad(e, "sync");
   S.ready = true;
   return VISTIO_OK;
@@ -2113,7 +2118,7 @@ vistio_status ensure_self_contact(const BatchDev&, SelfContactDev& S, const std:
     tris.push_back({s->setup.tris.data(), s->setup.nt});
     nverts.push_back(s->setup.nv);
   }
-  return self_build(S, tris, nverts, vbase, T, st, err);
+  return self_build(S, tris, nverts, vbase, T, true, st, err);
 }
 
 vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* px, const float* py,
@@ -2145,33 +2150,31 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
   SelfContactDev S;
   std::vector<std::pair<const uint32_t*, uint32_t>> tl{{tris, nt}};
   std::vector<uint32_t> nvs{nv}, vb{0};
-  vistio_status r = self_build(S, tl, nvs, vb, nt, st, err);
+  vistio_status r = self_build(S, tl, nvs, vb, nt, false, st, err);
   if (r != VISTIO_OK) return r;
   launch_self_sort(d, S.view(), uint32_t(ch.size()), st);
   launch_self_boxes(d, S.view(), uint32_t(ch.size()), margin, st);
-  k_self_count<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
-  k_scan_local<<<S.scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
-  k_scan_sums<<<1, kScanBlock, 0, st>>>(S.block_sums, S.scan_blocks, S.npairs);
-  k_scan_add<<<S.scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
+  k_self_pairs<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
   uint32_t total = 0;
   CU(cudaMemcpyAsync(&total, S.npairs, 4, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
-  if (total > S.pair_cap) {  // grow and recount
+  *count = total;
+  if (!pairs || total == 0) return VISTIO_OK;
+  if (total > S.pair_cap) {  // grow and find them again
     cudaFreeAsync(S.pairs, st);
     S.pairs = nullptr;
     S.pair_cap = total;
     CU(cudaMallocAsync(reinterpret_cast<void**>(&S.pairs), uint64_t(total) * sizeof(uint2), st));
+    CU(cudaMemsetAsync(S.npairs, 0, 4, st));
+    k_self_pairs<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
   }
-  k_self_write<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
+  DevBuf<uint32_t> row;
+  CU(row.alloc(total, st));
+  launch_sort_pairs(S.view(), nt, total, row.p, st);
   CU(cudaGetLastError());
-  std::vector<uint2> hp(total);
-  if (total) CU(cudaMemcpyAsync(hp.data(), S.pairs, uint64_t(total) * sizeof(uint2), cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(pairs, S.pairs, std::min<uint64_t>(total, cap) * sizeof(uint2), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
-  std::sort(hp.begin(), hp.end(), [](uint2 a, uint2 b) { return a.x != b.x ? a.x < b.x : a.y < b.y; });
-  *count = total;
-  if (pairs)
-    for (uint64_t k = 0; k < total && k < cap; ++k) { pairs[2 * k] = hp[k].x; pairs[2 * k + 1] = hp[k].y; }
-  if (pairs && total > cap) return fail(ctx, VISTIO_ERR_CAPACITY, "pair buffer too small");
+  if (total > cap) return fail(ctx, VISTIO_ERR_CAPACITY, "pair buffer too small");
   return VISTIO_OK;
 }
 
@@ -2259,7 +2262,7 @@ vistio_status ccd_hits_impl(vistio_ctx* ctx, uint32_t nv, const float* p0, const
 // not stored in spatial order.
 //
 // The region is sized for meshes of up to kNaMaxTris triangles and kNaMaxVerts
-// vertices and for up to kNaMaxPairs candidate pairs (about 16 MB); larger
+// vertices and for up to kNaMaxPairs candidate pairs (about 20 MB); larger
 // inputs are rejected with VISTIO_ERR_CAPACITY before any device work. There
 // is one region per device, so calls on the same device must not overlap:
 // two of them in flight at once (two threads, or two contexts' streams)
@@ -2297,7 +2300,8 @@ struct NaLayout {
   static constexpr uint64_t block_sums = cnt + na_up(4ull * kNaMaxTris);
   static constexpr uint64_t npairs = block_sums + na_up(4ull * kNaScanBlocks);  // [count, overflow]: zeroed
   static constexpr uint64_t pairs = npairs + na_up(8);
-  static constexpr uint64_t bytes = pairs + na_up(8ull * kNaMaxPairs);
+  static constexpr uint64_t row = pairs + na_up(8ull * kNaMaxPairs);  // sorting the pairs
+  static constexpr uint64_t bytes = row + na_up(4ull * kNaMaxPairs);
 };
 }  // namespace vistio_na
 
@@ -2338,9 +2342,6 @@ __global__ void k_na_pack(const float* __restrict__ x, const float* __restrict__
     }
   }
 }
-
-struct NaPair { uint32_t a, b; };
-static_assert(sizeof(NaPair) == 8, "pairs are two packed u32");
 
 vistio_status broadphase_pairs_noalloc_impl(vistio_ctx* ctx, uint32_t nv, const float* px, const float* py,
                                             const float* pz, uint32_t nt, const uint32_t* tris, float margin,
@@ -2412,10 +2413,7 @@ vistio_status broadphase_pairs_noalloc_impl(vistio_ctx* ctx, uint32_t nv, const 
                                          reinterpret_cast<int4*>(at(NaLayout::chunks)), nchunks);
   S.tall = I.nlevels > kLeafLevels + 1;
   launch_self_boxes(d, S, nchunks, margin, st);
-  k_self_count<<<nchunks, kElemThreads, 0, st>>>(d, S);
-  k_scan_local<<<scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
-  k_scan_sums<<<1, kScanBlock, 0, st>>>(S.block_sums, scan_blocks, S.npairs);
-  k_scan_add<<<scan_blocks, kScanBlock, 0, st>>>(S.cnt, nt, S.block_sums);
+  k_self_pairs<<<nchunks, kElemThreads, 0, st>>>(d, S);
   CU(cudaGetLastError());
   uint32_t total = 0;
   CU(cudaMemcpyAsync(&total, S.npairs, 4, cudaMemcpyDeviceToHost, st));
@@ -2426,15 +2424,11 @@ vistio_status broadphase_pairs_noalloc_impl(vistio_ctx* ctx, uint32_t nv, const 
                 "more than 1048576 candidate pairs: beyond the allocation-free broad phase; use vistio_broadphase_pairs");
   if (!pairs) return VISTIO_OK;  // size query
   if (total > cap) return fail(ctx, VISTIO_ERR_CAPACITY, "pair buffer too small");
-  k_self_write<<<nchunks, kElemThreads, 0, st>>>(d, S);
+  if (!total) return VISTIO_OK;
+  launch_sort_pairs(S, nt, total, reinterpret_cast<uint32_t*>(at(NaLayout::row)), st);
   CU(cudaGetLastError());
-  uint32_t status = 0;
-  if (total) CU(cudaMemcpyAsync(pairs, S.pairs, 8ull * total, cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(&status, d.status, 4, cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(pairs, S.pairs, 8ull * total, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
-  if (status & 2u) return fail(ctx, VISTIO_ERR_CAPACITY, "candidate pairs exceeded the scratch");
-  NaPair* P = reinterpret_cast<NaPair*>(pairs);
-  std::sort(P, P + total, [](const NaPair& u, const NaPair& v) { return u.a != v.a ? u.a < v.a : u.b < v.b; });
   return VISTIO_OK;
 }
 }  // namespace vistio_na
