@@ -301,42 +301,61 @@ __device__ __forceinline__ bool box_overlap(float4 amn, float4 amx, float4 bmn, 
   return amn.x <= bmx.x && amx.x >= bmn.x && amn.y <= bmx.y && amx.y >= bmn.y && amn.z <= bmx.z && amx.z >= bmn.z;
 }
 
-// Traversal for leaf i: visits subtrees holding leaves > i whose boxes overlap,
-// and writes the found pairs from out[base] on, up to cap of them. Returns how
-// many there are.
-__device__ uint32_t self_traverse(const SelfContactView& S, const SelfInst& I, uint32_t i, uint32_t base, uint2* out,
-                                  uint32_t cap) {
+// Traversal for leaf i: from the nodes k0, k0 + step, ... of level l0, the
+// subtrees holding leaves > i whose boxes overlap leaf i's; the found pairs go to
+// out[base] on, up to cap of them. Returns how many there are. A popped node
+// overlaps; its two children's boxes (neighbours in memory) are loaded and
+// tested together, so a level costs one round trip.
+__device__ uint32_t self_traverse(const SelfContactView& S, const SelfInst& I, uint32_t i, uint32_t l0, uint32_t k0,
+                                  uint32_t step, uint32_t base, uint2* out, uint32_t cap) {
   const float4* mn = S.box_min + I.box_base;
   const float4* mx = S.box_max + I.box_base;
-  float4 qmn = mn[i], qmx = mx[i];
-  uint32_t stack[64];
-  int sp = 0;
-  stack[sp++] = ((I.nlevels - 1) << 26) | 0u;  // (level, index) packed; index < 2^26
+  const float4 qmn = mn[i], qmx = mx[i];
+  uint32_t stack[32];  // (level, index) packed; index < 2^26; at most one entry waits per level
   uint32_t found = 0;
-  while (sp > 0) {
-    uint32_t code = stack[--sp];
-    uint32_t l = code >> 26, k = code & ((1u << 26) - 1);
-    uint64_t hi = (uint64_t(k) + 1) << l;  // one past the last leaf of the node
-    if (hi <= uint64_t(i) + 1) continue;
-    uint32_t o = I.lvl_off[l] + k;
-    if (!box_overlap(qmn, qmx, mn[o], mx[o])) continue;
-    if (l == 0) {
-      uint32_t slot = base + found;
-      if (slot < cap) {
-        uint32_t a = I.tbase + i, b = I.tbase + k;
-        if (S.leaf_tri) {
-          a = S.leaf_tri[a];
-          b = S.leaf_tri[b];
-        }
-        out[slot] = make_uint2(min(a, b), max(a, b));
-      }
-      ++found;
+  auto reaches = [&](uint32_t l, uint32_t k) { return ((uint64_t(k) + 1) << l) > uint64_t(i) + 1; };
+  auto leaf = [&](uint32_t k) {
+    const uint32_t slot = base + found++;
+    if (slot >= cap) return;
+    uint32_t a = I.tbase + i, b = I.tbase + k;
+    if (S.leaf_tri) {
+      a = S.leaf_tri[a];
+      b = S.leaf_tri[b];
+    }
+    out[slot] = make_uint2(min(a, b), max(a, b));
+  };
+  for (uint32_t start = k0; start < I.lvl_cnt[l0]; start += step) {
+    if (!reaches(l0, start)) continue;
+    const uint32_t o0 = I.lvl_off[l0] + start;
+    if (!box_overlap(qmn, qmx, mn[o0], mx[o0])) continue;
+    if (l0 == 0) {
+      leaf(start);
       continue;
     }
-    // children (l-1, 2k) and (l-1, 2k+1); the right child may not exist.
-    // The stack never holds more than two entries per level (< 64).
-    if (2 * k + 1 < I.lvl_cnt[l - 1]) stack[sp++] = ((l - 1) << 26) | (2 * k + 1);
-    stack[sp++] = ((l - 1) << 26) | (2 * k);
+    int sp = 0;
+    uint32_t l = l0, k = start;
+    for (;;) {
+      // children (l-1, 2k) and (l-1, 2k+1); the right child may not exist
+      const uint32_t kl = 2 * k, kr = kl + 1, o = I.lvl_off[l - 1] + kl;
+      bool left = reaches(l - 1, kl), right = kr < I.lvl_cnt[l - 1] && reaches(l - 1, kr);
+      float4 amn, amx, bmn, bmx;
+      if (left) { amn = mn[o]; amx = mx[o]; }
+      if (right) { bmn = mn[o + 1]; bmx = mx[o + 1]; }
+      left = left && box_overlap(qmn, qmx, amn, amx);
+      right = right && box_overlap(qmn, qmx, bmn, bmx);
+      if (l == 1) {
+        if (left) leaf(kl);
+        if (right) leaf(kr);
+      } else if (left || right) {
+        if (left && right) stack[sp++] = ((l - 1) << 26) | kr;
+        l = l - 1;
+        k = left ? kl : kr;
+        continue;
+      }
+      if (!sp) break;
+      l = stack[--sp] >> 26;
+      k = stack[sp] & ((1u << 26) - 1);
+    }
   }
   return found;
 }
@@ -392,18 +411,30 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_add(uint32_t* v, uint32_t n
 // keeps its first kPairBuf pairs in a local buffer while it walks the tree,
 // its warp takes slots for all of them with one atomic, and a thread that
 // found more walks the tree again to write them all.
+//
+// A traversal is a chain of round trips, and a single garment's leaves do not
+// fill the chip: so it starts from all nodes of a level below the root, whose
+// tests do not depend on each other, and G threads share a leaf's. Two contact
+// steps of a folded ribbon of 32,000 triangles with one thread per leaf from the
+// root 4.80 ms; G = 4 from the third level below the root 4.30, from the fifth
+// 4.00, from the seventh 3.83 (G = 8, fifth: 3.96). A step of 64 drapes (795,264
+// triangles; the chip is full): one thread per leaf from the root 20.4 ms, from the
+// fifth level 19.9; G = 2 from the third 20.4.
 constexpr uint32_t kPairBuf = 24;
-__global__ void __launch_bounds__(256) k_self_pairs(BatchDev B, SelfContactView S) {
+constexpr uint64_t kSharedLeaves = 148 * 2048 / 4;
+template <uint32_t G> __global__ void __launch_bounds__(256) k_self_pairs(BatchDev B, SelfContactView S) {
   pdl_begin();
-  const int4 ch = B.tri_chunks[blockIdx.x];
-  const bool live = (int)threadIdx.x < ch.z && !(B.prm->ipc && B.red[ch.x].al_done);
+  const int4 ch = B.tri_chunks[blockIdx.x / G];
+  const uint32_t at = (blockIdx.x % G * 256 + threadIdx.x) / G;
+  const bool live = (int)at < ch.z && !(B.prm->ipc && B.red[ch.x].al_done);
   const uint32_t lane = threadIdx.x & 31u;
   uint2 buf[kPairBuf];
   uint32_t found = 0, i = 0;
   const SelfInst& I = S.inst[ch.x];  // read in place (cached): the block's threads share it
+  const uint32_t top = I.nlevels - 1, l0 = top - min(top, G == 1 ? 5u : 7u);
   if (live) {
-    i = uint32_t(ch.y) + threadIdx.x - I.tbase;
-    found = self_traverse(S, I, i, 0, buf, kPairBuf);
+    i = uint32_t(ch.y) + at - I.tbase;
+    found = self_traverse(S, I, i, l0, threadIdx.x % G, G, 0, buf, kPairBuf);
   }
   uint32_t incl = found;
 #pragma unroll
@@ -424,8 +455,15 @@ __global__ void __launch_bounds__(256) k_self_pairs(BatchDev B, SelfContactView 
     for (uint32_t j = 0; j < found; ++j)
       if (uint64_t(base) + j < cap) S.pairs[base + j] = buf[j];
   } else {
-    self_traverse(S, I, i, base, S.pairs, uint32_t(cap));
+    self_traverse(S, I, i, l0, threadIdx.x % G, G, base, S.pairs, uint32_t(cap));
   }
+}
+
+// Threads per leaf: as many as keep the resident threads (148 SMs x 2048) busy.
+inline uint32_t launch_self_pairs(const BatchDev& d, const SelfContactView& S, uint32_t n_tri_chunks, cudaStream_t st) {
+  if (S.T <= kSharedLeaves) launch_pdl(k_self_pairs<4>, 4 * n_tri_chunks, 256, 0, st, d, S);
+  else launch_pdl(k_self_pairs<1>, n_tri_chunks, 256, 0, st, d, S);
+  return 1;
 }
 
 // The pairs (a < b) in ascending order, on the device: counted per first
@@ -1053,7 +1091,7 @@ inline uint32_t launch_self_detect(const BatchDev& d, const SelfContactView& S, 
                                    uint32_t n_tri_chunks, int mode, cudaStream_t st) {
   launch_pdl(k_clear_grad, n_vtx_chunks, 256, 0, st, d);
   uint32_t nl = 3 + launch_self_boxes(d, S, n_tri_chunks, -1.f, st);  // margin: StepParams::thickness
-  launch_pdl(k_self_pairs, n_tri_chunks, 256, 0, st, d, S);
+  launch_self_pairs(d, S, n_tri_chunks, st);
   if (S.vt_on && mode == 0) {  // the pass's CCD tests
     launch_pdl(k_self_vt, 6 * 148, 256, 0, st, d, S);  // 40 registers: six blocks per SM
     ++nl;

@@ -2154,7 +2154,7 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
   if (r != VISTIO_OK) return r;
   launch_self_sort(d, S.view(), uint32_t(ch.size()), st);
   launch_self_boxes(d, S.view(), uint32_t(ch.size()), margin, st);
-  k_self_pairs<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
+  launch_self_pairs(d, S.view(), uint32_t(ch.size()), st);
   uint32_t total = 0;
   CU(cudaMemcpyAsync(&total, S.npairs, 4, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
@@ -2166,7 +2166,7 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
     S.pair_cap = total;
     CU(cudaMallocAsync(reinterpret_cast<void**>(&S.pairs), uint64_t(total) * sizeof(uint2), st));
     CU(cudaMemsetAsync(S.npairs, 0, 4, st));
-    k_self_pairs<<<uint32_t(ch.size()), 256, 0, st>>>(d, S.view());
+    launch_self_pairs(d, S.view(), uint32_t(ch.size()), st);
   }
   DevBuf<uint32_t> row;
   CU(row.alloc(total, st));
@@ -2413,7 +2413,7 @@ vistio_status broadphase_pairs_noalloc_impl(vistio_ctx* ctx, uint32_t nv, const 
                                          reinterpret_cast<int4*>(at(NaLayout::chunks)), nchunks);
   S.tall = I.nlevels > kLeafLevels + 1;
   launch_self_boxes(d, S, nchunks, margin, st);
-  k_self_pairs<<<nchunks, kElemThreads, 0, st>>>(d, S);
+  launch_self_pairs(d, S, nchunks, st);
   CU(cudaGetLastError());
   uint32_t total = 0;
   CU(cudaMemcpyAsync(&total, S.npairs, 4, cudaMemcpyDeviceToHost, st));
