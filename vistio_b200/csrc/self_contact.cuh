@@ -66,7 +66,7 @@ struct SelfContactView {
   // times per test on a cloth mesh. The list keeps (v, B) only from the pair
   // whose A is the lowest-numbered triangle around v with a box overlapping
   // B's, which is the first pair the broad phase holds for that test. Built
-  // by the detect that opens an AL pass; the pass's CCDs read it.
+  // when an AL pass opens; the pass's CCDs read it.
   uint32_t* leaf_of;     // global triangle -> its leaf in its garment's tree (null: no list)
   uint2* vt;             // (vertex, triangle), global ids
   uint32_t* nvt;         // [0] tests, [1] overflow: the CCD then runs over the pairs
@@ -535,8 +535,9 @@ __global__ void __launch_bounds__(256) k_self_vt(BatchDev B, SelfContactView S) 
     const uint32_t k = k0 + lane;
     uint2 keep[6];
     uint32_t c = 0;
-    if (k < np) {
-      const uint2 pr = S.pairs[k];
+    const uint2 pr = k < np ? S.pairs[k] : make_uint2(0u, 0u);
+    // (a garment may be done since the detect whose pairs these are)
+    if (k < np && !B.red[S.tri_inst[pr.x]].al_done) {
       const uint32_t inst = S.tri_inst[pr.x];
       const InstDev I = B.inst[inst];
       const uint32_t box_base = S.inst[inst].box_base;
@@ -1086,18 +1087,22 @@ inline uint32_t launch_self_boxes(const BatchDev& d, const SelfContactView& S, u
   return S.tall ? 2 : 1;
 }
 
-// Returns the kernels launched.
+// The self-contact part of a detect: boxes, candidate pairs and the gradient of
+// their contacts (mode 1 also counts them). Returns the launches.
 inline uint32_t launch_self_detect(const BatchDev& d, const SelfContactView& S, uint32_t n_vtx_chunks,
                                    uint32_t n_tri_chunks, int mode, cudaStream_t st) {
   launch_pdl(k_clear_grad, n_vtx_chunks, 256, 0, st, d);
-  uint32_t nl = 3 + launch_self_boxes(d, S, n_tri_chunks, -1.f, st);  // margin: StepParams::thickness
+  const uint32_t nl = 3 + launch_self_boxes(d, S, n_tri_chunks, -1.f, st);  // margin: StepParams::thickness
   launch_self_pairs(d, S, n_tri_chunks, st);
-  if (S.vt_on && mode == 0) {  // the pass's CCD tests
-    launch_pdl(k_self_vt, 6 * 148, 256, 0, st, d, S);  // 40 registers: six blocks per SM
-    ++nl;
-  }
   launch_pdl(k_self_grad, 3 * 148, kGradThreads, 0, st, d, S, mode);
   return nl;
+}
+
+// The pass's CCD tests from the last detect's pairs. Returns the launches.
+inline uint32_t launch_self_tests(const BatchDev& d, const SelfContactView& S, cudaStream_t st) {
+  if (!S.vt_on) return 0;
+  launch_pdl(k_self_vt, 6 * 148, 256, 0, st, d, S);  // 40 registers: six blocks per SM
+  return 1;
 }
 
 // Sorts the n pairs found over nt triangles (row: room for n).

@@ -937,12 +937,14 @@ uint32_t launch_plain_iteration(vistio_batch* b, cudaStream_t st, int do_update,
   return n + launch_solve(b, st, do_update, refine, false);
 }
 
-// One Augmented-Lagrangian pass of an IPC step. Returns the launches.
+// One Augmented-Lagrangian pass of an IPC step. Returns the launches. It opens
+// with the contacts at the positions where the last pass ended (its closing
+// self-contact detect, or for the first pass one before the loop).
 uint32_t launch_al_pass(vistio_batch* b, bool self, cudaGraphConditionalHandle again, cudaStream_t st) {
   const uint32_t small_grid = (b->ninst + 127) / 128;
   uint32_t L = 5;
   k_al_begin<<<small_grid, 128, 0, st>>>(b->dev, b->ninst);  // first in the loop's body: no kernel to overlap
-  if (self) L += launch_self_detect(b->dev, b->self.view(), b->n_vtx_chunks, b->n_tri_chunks, 0, st);
+  if (self) L += launch_self_tests(b->dev, b->self.view(), st);
   launch_pdl(k_detect, b->n_vtx_chunks, kElemThreads, 0, st, b->dev, 0);
   for (uint32_t it = 0; it < b->cfg.max_iterations; ++it) {
     // With backtracking (alpha < 1) part of each sweep's error stays in x:
@@ -981,7 +983,10 @@ vistio_status capture(vistio_batch* b, bool ipc, bool self, cudaGraphExec_t* out
     launch_pdl(k_finalize, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
   } else {
     if (b->cfg.al_max_iterations) {
-      if (self) L += launch_self_sort(b->dev, b->self.view(), b->n_tri_chunks, st);
+      if (self) {
+        L += launch_self_sort(b->dev, b->self.view(), b->n_tri_chunks, st);
+        L += launch_self_detect(b->dev, b->self.view(), b->n_vtx_chunks, b->n_tri_chunks, 0, st);
+      }
       cudaStreamCaptureStatus status;
       const cudaGraphNode_t* deps = nullptr;
       size_t ndeps = 0;
