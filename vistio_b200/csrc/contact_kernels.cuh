@@ -212,13 +212,12 @@ __device__ __forceinline__ void collider_ccd(const BatchDev& B, uint32_t chunk) 
   const StepParams& P = *B.prm;
   InstRed& R = B.red[ch.x];
   if (R.al_done) return;
-  const InstDev I = B.inst[ch.x];
   float toi = 1.f;
   double gdd = 0.0;
   if ((int)threadIdx.x < ch.z) {
     uint32_t g = uint32_t(ch.y) + threadIdx.x;
     float4 x0 = B.pos[g];
-    float4 d = B.Y[I.vbase + B.perm_local[g]];
+    float4 d = B.T[g];
     float3 x1 = make_float3(x0.x + d.x, x0.y + d.y, x0.z + d.z);
     if (P.has_ground) {
       float y0 = x0.y, y1 = x1.y, h = P.ground_h;
@@ -471,7 +470,7 @@ __global__ void __launch_bounds__(256) k_ipc_update(BatchDev B) {
   if ((int)threadIdx.x >= ch.z) return;
   uint32_t g = uint32_t(ch.y) + threadIdx.x;
   if (B.pinned[g]) return;
-  float4 d = B.Y[I.vbase + B.perm_local[g]];
+  float4 d = B.T[g];
   float4 x = B.pos[g];
   x.x += alpha * d.x; x.y += alpha * d.y; x.z += alpha * d.z;
   B.pos[g] = x;

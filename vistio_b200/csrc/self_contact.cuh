@@ -998,12 +998,11 @@ __device__ __noinline__ void ccd_pairs(const BatchDev& B, const SelfContactView&
     uint32_t inst = S.tri_inst[pr.x];
     InstRed& R = B.red[inst];
     if (R.al_done) continue;
-    const InstDev I = B.inst[inst];
     uint4 A = B.tri_idx[pr.x], Bt = B.tri_idx[pr.y];
     uint32_t av[3] = {A.x, A.y, A.z}, bv[3] = {Bt.x, Bt.y, Bt.z};
     auto P0 = [&](uint32_t v) { return ld3(B.pos, v); };
     auto P1 = [&](uint32_t v) {
-      float4 x = B.pos[v], d = B.Y[I.vbase + B.perm_local[v]];
+      float4 x = B.pos[v], d = B.T[v];
       return mk<float>(x.x + d.x, x.y + d.y, x.z + d.z);
     };
     float best = 2.f;
@@ -1041,11 +1040,10 @@ __global__ void __launch_bounds__(256, 6) k_ccd_self(const __grid_constant__ Bat
     const uint32_t inst = S.tri_inst[tst.y];
     InstRed& R = B.red[inst];
     if (R.al_done) continue;
-    const uint32_t vbase = B.inst[inst].vbase;
     const uint4 T = B.tri_idx[tst.y];
     auto P0 = [&](uint32_t v) { return ld3(B.pos, v); };
     auto P1 = [&](uint32_t v) {
-      float4 x = B.pos[v], d = B.Y[vbase + B.perm_local[v]];
+      float4 x = B.pos[v], d = B.T[v];
       return mk<float>(x.x + d.x, x.y + d.y, x.z + d.z);
     };
     const float t = vt_ccd<float>(P0(tst.x), P1(tst.x), P0(T.x), P1(T.x), P0(T.y), P1(T.y), P0(T.z), P1(T.z));
