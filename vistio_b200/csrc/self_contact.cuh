@@ -5,9 +5,8 @@
 // and refits it otherwise (crates/vistio-contact/src/bvh.rs:122-373). Here each
 // garment's triangles, ordered by the Morton code of their centroid, are the
 // leaves of an implicit balanced binary tree: node (l, i) bounds leaves
-// [i 2^l, (i+1) 2^l). A node's leaf range is known from its position, so the
-// traversal for leaf i skips every subtree whose leaves are all <= i and emits
-// exactly the pairs (i < j) whose inflated AABBs overlap: the complete candidate
+// [i 2^l, (i+1) 2^l). The traversal for leaf i covers exactly the leaves j > i and
+// emits the pairs (i < j) whose inflated AABBs overlap: the complete candidate
 // set, whatever the order of the leaves. So a step sorts once, at its predicted
 // positions, and its detects only refit the boxes.
 #pragma once
@@ -301,19 +300,23 @@ __device__ __forceinline__ bool box_overlap(float4 amn, float4 amx, float4 bmn, 
   return amn.x <= bmx.x && amx.x >= bmn.x && amn.y <= bmx.y && amx.y >= bmn.y && amn.z <= bmx.z && amx.z >= bmn.z;
 }
 
-// Traversal for leaf i: from the nodes k0, k0 + step, ... of level l0, the
-// subtrees holding leaves > i whose boxes overlap leaf i's; the found pairs go to
-// out[base] on, up to cap of them. Returns how many there are. A popped node
-// overlaps; its two children's boxes (neighbours in memory) are loaded and
-// tested together, so a level costs one round trip.
-__device__ uint32_t self_traverse(const SelfContactView& S, const SelfInst& I, uint32_t i, uint32_t l0, uint32_t k0,
-                                  uint32_t step, uint32_t base, uint2* out, uint32_t cap) {
+// Traversal for leaf i, thread g of the G that share it: the leaves above i are
+// those below the right siblings of the nodes on its path to the root. Those
+// whose boxes overlap leaf i's go to out[base] on, up to cap of them. Returns how
+// many there are. A node taken from the stack overlaps; its two children's boxes
+// (neighbours in memory) are loaded and tested together. Threads that share a
+// leaf start, in place of the siblings of the kWideLevels highest levels, from
+// all nodes right of the path on the level below them: more tests, but
+// independent ones.
+constexpr uint32_t kWideLevels = 8;
+template <uint32_t G>
+__device__ uint32_t self_traverse(const SelfContactView& S, const SelfInst& I, uint32_t i, uint32_t g, uint32_t base,
+                                  uint2* out, uint32_t cap) {
   const float4* mn = S.box_min + I.box_base;
   const float4* mx = S.box_max + I.box_base;
   const float4 qmn = mn[i], qmx = mx[i];
   uint32_t stack[32];  // (level, index) packed; index < 2^26; at most one entry waits per level
   uint32_t found = 0;
-  auto reaches = [&](uint32_t l, uint32_t k) { return ((uint64_t(k) + 1) << l) > uint64_t(i) + 1; };
   auto leaf = [&](uint32_t k) {
     const uint32_t slot = base + found++;
     if (slot >= cap) return;
@@ -324,38 +327,52 @@ __device__ uint32_t self_traverse(const SelfContactView& S, const SelfInst& I, u
     }
     out[slot] = make_uint2(min(a, b), max(a, b));
   };
-  for (uint32_t start = k0; start < I.lvl_cnt[l0]; start += step) {
-    if (!reaches(l0, start)) continue;
-    const uint32_t o0 = I.lvl_off[l0] + start;
-    if (!box_overlap(qmn, qmx, mn[o0], mx[o0])) continue;
-    if (l0 == 0) {
-      leaf(start);
-      continue;
+  auto below = [&](uint32_t l, uint32_t k) {
+    const uint32_t o0 = I.lvl_off[l] + k;
+    if (!box_overlap(qmn, qmx, mn[o0], mx[o0])) return;
+    if (l == 0) {
+      leaf(k);
+      return;
     }
     int sp = 0;
-    uint32_t l = l0, k = start;
     for (;;) {
       // children (l-1, 2k) and (l-1, 2k+1); the right child may not exist
-      const uint32_t kl = 2 * k, kr = kl + 1, o = I.lvl_off[l - 1] + kl;
-      bool left = reaches(l - 1, kl), right = kr < I.lvl_cnt[l - 1] && reaches(l - 1, kr);
-      float4 amn, amx, bmn, bmx;
-      if (left) { amn = mn[o]; amx = mx[o]; }
-      if (right) { bmn = mn[o + 1]; bmx = mx[o + 1]; }
-      left = left && box_overlap(qmn, qmx, amn, amx);
-      right = right && box_overlap(qmn, qmx, bmn, bmx);
-      if (l == 1) {
+      const uint32_t kl = 2 * k, o = I.lvl_off[l - 1] + kl, two = kl + 1 < I.lvl_cnt[l - 1];
+      const bool left = box_overlap(qmn, qmx, mn[o], mx[o]);
+      const bool right = box_overlap(qmn, qmx, mn[o + two], mx[o + two]) && two;
+      --l;
+      if (l == 0) {
         if (left) leaf(kl);
-        if (right) leaf(kr);
+        if (right) leaf(kl + 1);
       } else if (left || right) {
-        if (left && right) stack[sp++] = ((l - 1) << 26) | kr;
-        l = l - 1;
-        k = left ? kl : kr;
+        if (left && right) stack[sp++] = (l << 26) | (kl + 1);
+        k = left ? kl : kl + 1;
         continue;
       }
       if (!sp) break;
       l = stack[--sp] >> 26;
       k = stack[sp] & ((1u << 26) - 1);
     }
+  };
+  // the starts: entries of level `wide` (G > 1), then the siblings below it
+  const uint32_t top = I.nlevels - 1, wide = G > 1 && top > kWideLevels ? top - kWideLevels : top;
+  uint32_t l = wide, k = G > 1 ? (i >> wide) + 1 + g : I.lvl_cnt[wide];
+  for (;;) {
+    if (l == wide && k < I.lvl_cnt[wide]) {
+      below(l, k);
+      k += G;
+      continue;
+    }
+    if (l == wide) {  // on to the siblings: this thread's levels
+      if (wide == 0) break;
+      l = (wide - 1) - g % G;
+      if (g >= wide) break;
+    } else {
+      if (l < G) break;
+      l -= G;
+    }
+    const uint32_t sib = (i >> l) + 1;
+    if ((sib & 1u) && sib < I.lvl_cnt[l]) below(l, sib);
   }
   return found;
 }
@@ -412,16 +429,15 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_add(uint32_t* v, uint32_t n
 // its warp takes slots for all of them with one atomic, and a thread that
 // found more walks the tree again to write them all.
 //
-// A traversal is a chain of round trips, and a single garment's leaves do not
-// fill the chip: so it starts from all nodes of a level below the root, whose
-// tests do not depend on each other, and G threads share a leaf's. Two contact
-// steps of a folded ribbon of 32,000 triangles with one thread per leaf from the
-// root 4.80 ms; G = 4 from the third level below the root 4.30, from the fifth
-// 4.00, from the seventh 3.83 (G = 8, fifth: 3.96). A step of 64 drapes (795,264
-// triangles; the chip is full): one thread per leaf from the root 20.4 ms, from the
-// fifth level 19.9; G = 2 from the third 20.4.
+// G threads share a leaf where the leaves alone do not fill the chip (a
+// traversal is a chain of round trips). Two contact steps of a folded ribbon of
+// 32,000 triangles, from the root and one thread per leaf 4.80 ms; the siblings
+// alone with G = 1 / 4 / 8 4.77 / 4.11 / 4.08; with kWideLevels 7 and G = 4 / 8
+// 3.88 / 3.75, 8 and 8 3.70. A step of 64 drapes (795,264 triangles: the chip is
+// full, and it is bound by instructions at 10 of 32 threads) from the root 18.1 ms,
+// from the siblings with G = 1 / 2 / 4 17.5 / 17.8 / 18.3.
 constexpr uint32_t kPairBuf = 24;
-constexpr uint64_t kSharedLeaves = 148 * 2048 / 4;
+constexpr uint64_t kSharedLeaves = 148 * 2048 / 4;  // two rounds of eight threads per leaf
 template <uint32_t G> __global__ void __launch_bounds__(256) k_self_pairs(BatchDev B, SelfContactView S) {
   pdl_begin();
   const int4 ch = B.tri_chunks[blockIdx.x / G];
@@ -431,10 +447,9 @@ template <uint32_t G> __global__ void __launch_bounds__(256) k_self_pairs(BatchD
   uint2 buf[kPairBuf];
   uint32_t found = 0, i = 0;
   const SelfInst& I = S.inst[ch.x];  // read in place (cached): the block's threads share it
-  const uint32_t top = I.nlevels - 1, l0 = top - min(top, G == 1 ? 5u : 7u);
   if (live) {
     i = uint32_t(ch.y) + at - I.tbase;
-    found = self_traverse(S, I, i, l0, threadIdx.x % G, G, 0, buf, kPairBuf);
+    found = self_traverse<G>(S, I, i, threadIdx.x % G, 0, buf, kPairBuf);
   }
   uint32_t incl = found;
 #pragma unroll
@@ -455,13 +470,12 @@ template <uint32_t G> __global__ void __launch_bounds__(256) k_self_pairs(BatchD
     for (uint32_t j = 0; j < found; ++j)
       if (uint64_t(base) + j < cap) S.pairs[base + j] = buf[j];
   } else {
-    self_traverse(S, I, i, l0, threadIdx.x % G, G, base, S.pairs, uint32_t(cap));
+    self_traverse<G>(S, I, i, threadIdx.x % G, base, S.pairs, uint32_t(cap));
   }
 }
 
-// Threads per leaf: as many as keep the resident threads (148 SMs x 2048) busy.
 inline uint32_t launch_self_pairs(const BatchDev& d, const SelfContactView& S, uint32_t n_tri_chunks, cudaStream_t st) {
-  if (S.T <= kSharedLeaves) launch_pdl(k_self_pairs<4>, 4 * n_tri_chunks, 256, 0, st, d, S);
+  if (S.T <= kSharedLeaves) launch_pdl(k_self_pairs<8>, 8 * n_tri_chunks, 256, 0, st, d, S);
   else launch_pdl(k_self_pairs<1>, n_tri_chunks, 256, 0, st, d, S);
   return 1;
 }
