@@ -25,7 +25,7 @@
 // warp. A chunk's sum is one chain of fused multiply-adds from zero in ascending
 // column order, and a row's chunks are added in ascending order. Neither depends
 // on who runs the task, so every schedule gives the same bits:
-//   warp items   a supernode of at most 32 columns, run by one warp;
+//   warp items   a supernode of at most 64 columns, run by one warp;
 //   block items  some tiles of one supernode, their tasks shared by the warps.
 // W is stored twice (tiles of its rows for the forward product, of its columns
 // for the backward one): the same bytes are read either way.
@@ -48,19 +48,22 @@ constexpr uint32_t kForms = 3;
 constexpr uint32_t kFormWarps[kForms] = {6, 8, 16};
 constexpr uint32_t kFormBlocks[kForms] = {5, 4, 2};
 constexpr uint32_t kTile = 32;      // rows of a tile and columns of a chunk
+constexpr uint32_t kWarpCols = 64;  // columns of a supernode that one warp may take
 constexpr uint32_t kMaxTasks = 32;  // tasks of an item whose chunks are shared
 // Columns of v staged at a time: what the blocks per SM leave room for. The
 // sixteen-warp form takes a supernode of up to 1024 in one piece, so that the
 // chunks of its tiles can be shared (97x97 sheet, root of 578 columns: 486 us
 // per step with 512, the root's tiles one warp each).
 __host__ __device__ constexpr uint32_t vec_cols(uint32_t warps) { return warps == 16 ? 1024 : 512; }
+static_assert(vec_cols(6) >= 6 * kWarpCols && vec_cols(8) >= 8 * kWarpCols && vec_cols(16) >= 16 * kWarpCols,
+              "the warps' own entries of v fit the block's");
 __host__ __device__ constexpr uint32_t level_smem(uint32_t warps) {
   return warps * kTile * kTile * 4 + vec_cols(warps) * 16 + kMaxTasks * kTile * 12;
 }
 // Default limit of s (s + m) for a warp item; vistio_batch_tune picks one per batch.
 constexpr uint32_t kWarpItemLimit = 6144;
 __host__ __device__ constexpr bool warp_item(uint32_t s, uint32_t m, uint32_t limit = kWarpItemLimit) {
-  return s <= kTile && uint64_t(s) * (s + m) <= limit;
+  return s <= kWarpCols && uint64_t(s) * (s + m) <= limit;
 }
 
 // One work item: some tiles of one supernode's product in one direction. All a
@@ -334,9 +337,9 @@ __device__ __forceinline__ void block_item(const BatchDev& B, const SweepItem& I
   if (warp < nt) out.put(B, I, total);
 }
 
-// One item of a supernode of at most 32 columns by one warp: a chunk of columns
-// at a time (forward there is one, backward one tile). v: 32 entries of the
-// warp's own.
+// One item of a supernode of at most kWarpCols columns by one warp: forward some
+// of its tiles, over its one or two chunks; backward one tile. v: kWarpCols
+// entries of the warp's own (backward a chunk at a time).
 template <int DIR, class Wait>
 __device__ __forceinline__ void warp_tiles(const BatchDev& B, const SweepItem& I, Stage& st, float4* v, Wait wait) {
   const Panel<DIR> M(B, I);
@@ -348,6 +351,7 @@ __device__ __forceinline__ void warp_tiles(const BatchDev& B, const SweepItem& I
     out.begin(B, I, (I.tile0 + t) * kTile + lane);
     for (uint32_t ch = 0; ch < all; ++ch) {
       const uint32_t nc = M.chunk(ch);
+      float4* vc = DIR == 0 ? v + ch * kTile : v;
       if (t == 0) {
         Entry<DIR> e;
         if (lane < nc) e.prepare(B, I, ch * kTile + lane);
@@ -355,13 +359,13 @@ __device__ __forceinline__ void warp_tiles(const BatchDev& B, const SweepItem& I
           st.wait(B.status);  // the copy in flight lands before the block ends
           return;
         }
-        __syncwarp();  // the last chunk's readers of v are done
-        if (lane < nc) v[lane] = e.get(B);
+        if (DIR == 1) __syncwarp();  // the last chunk's readers of v are done
+        if (lane < nc) vc[lane] = e.get(B);
         __syncwarp();
       }
       if (ch == 0) out.after(B, I);
       st.wait(B.status);
-      const float4 p = st.sum(v, M.width(I.tile0 + t), nc);
+      const float4 p = st.sum(vc, M.width(I.tile0 + t), nc);
       total = ch == 0 ? p : f4_add(total, p);
       if (ch + 1 < all) M.issue(st, I.tile0 + t, ch + 1);
       else if (t + 1 < I.ntiles) M.issue(st, I.tile0 + t + 1, 0);
@@ -403,7 +407,7 @@ k_level(BatchDev B, const SweepItem* __restrict__ items, uint32_t nblock, uint32
     return;
   }
   const SweepItem I = items[nblock + q];
-  warp_tiles<DIR>(B, I, st, v + warp * kTile, [&]() {
+  warp_tiles<DIR>(B, I, st, v + warp * kWarpCols, [&]() {
     pdl_begin();
     return !(B.prm->ipc && B.red[I.inst].al_done);
   });

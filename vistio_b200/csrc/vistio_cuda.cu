@@ -216,10 +216,15 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
 
 // Tasks (tile x chunk) that one phase can spread over the chip's resident warps
 // (148 SMs x 4 blocks x 8 warps). A phase of fewer is as long as its longest
-// item, so its items are cut to one task per warp; the items of a larger phase
-// grow with it, since every block item gathers its own v (up to kItemTasks).
+// item, so its items are cut to one task per warp; the block items of a larger
+// phase grow with it, since every one gathers its own v (up to kItemTasks; 512
+// sheets with 8 / 32 / 64: 14.21 / 12.40 / 12.36 ms per step). From kManyTasks on
+// a warp takes all tiles of its supernode (24 sheets, below the line: 1546 us so,
+// 1493 with a tile per warp) and supernodes of two chunks too (24 sheets 1590 us so,
+// 1546 with a block each; 512 sheets, above it, 12.4 ms so, 13.3 with a block each).
 constexpr uint64_t kPhaseTasks = 148 * 4 * 8;
-constexpr uint64_t kItemTasks = 32;
+constexpr uint64_t kManyTasks = 4 * kPhaseTasks;
+constexpr uint64_t kItemTasks = 64;
 
 // The sweeps' schedule for a warp-item limit, uploaded: every supernode's step
 // as work items (solve_kernels.cuh), in phases of independent supernodes.
@@ -259,11 +264,11 @@ cudaError_t schedule(vistio_batch* b, uint32_t limit, cudaStream_t st) {
     for (int pass = 0; pass < 2; ++pass)  // block items first
       for (uint32_t k : list) {
         const SnDev& S = b->sn_host[k];
-        const bool warp = warp_item(S.ncols, S.nrows, limit);
+        const bool warp = warp_item(S.ncols, S.nrows, limit) && (S.ncols <= kTile || tasks > kManyTasks);
         if (warp != (pass == 1)) continue;
         if (dir == 1 && S.nrows == 0) continue;  // a root's forward step is its solution
         const uint32_t tiles = tiles_in(S);
-        const uint32_t per = warp ? (tasks <= kPhaseTasks ? 1u : tiles)
+        const uint32_t per = warp ? (dir == 1 || tasks <= kManyTasks ? 1u : tiles)
                                   : std::max(1u, uint32_t(per_item / chunks_in(S)));
         for (uint32_t t = 0; t < tiles; t += per) {
           items.push_back(SweepItem{dir == 0 ? S.f_off : S.b_off, S.vbase + S.first, S.vbase, S.ncols, S.nrows, S.rows_off,
@@ -1575,8 +1580,8 @@ void* vistio_batch_stream(vistio_batch* b) { return b ? (void*)b->ctx->stream : 
 
 // Sweep autotuner. The candidates are the orders of the work (by height, by
 // depth, groups side by side) times the warp-item limits of s (s + m): 0 (every
-// supernode for a block) ... 2^30 (every one of at most kTile columns for a
-// warp), and for the grouped order the group limits.
+// supernode for a block) ... 2^30 (every one of at most kWarpCols columns
+// for a warp), and for the grouped order the group limits.
 static const uint32_t kTuneLimits[7] = {0u, 1024u, 2048u, 4096u, 6144u, 12288u, 1u << 30};
 // Group limits of the grouped kind's candidates: 0 takes the leaves only.
 static const uint32_t kGroupTuneLimits[7] = {0u, 64u, 128u, 256u, 512u, 1024u, 6144u};
