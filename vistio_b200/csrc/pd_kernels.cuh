@@ -587,16 +587,13 @@ __global__ void __launch_bounds__(256) k_accum(BatchDev B) {
   B.Y[p] = f4_add(B.Y[p], B.W[p]);
 }
 
-// After the sweeps: residual sums (pd_solver.rs:403-421) and, for the plain
-// step, x <- x + d, the pin reset (:429-435) and the ground clamp (:438); for
-// the IPC step, whose line search and update read d several times, d in vertex
-// order into T (the sweeps are done with their right-hand side).
+// After the sweeps of a plain step: residual sums (pd_solver.rs:403-421) and, with
+// do_update, x <- x + d, the pin reset (:429-435) and the ground clamp (:438).
 // add_w folds the last refinement correction into d.
 __device__ __forceinline__ void update_one(const BatchDev& B, const InstDev& I, uint32_t g, float4 d, float4 x,
                                            int do_update, int add_w, uint32_t row, double& dsq, double& nsq,
                                            bool& bad) {
   if (add_w) d = f4_add(d, B.W[row]);
-  if (!do_update) B.T[g] = d;
   dsq += double(d.x) * d.x + double(d.y) * d.y + double(d.z) * d.z;
   nsq += double(x.x) * x.x + double(x.y) * x.y + double(x.z) * x.z;
   bad = bad || !(isfinite(d.x) && isfinite(d.y) && isfinite(d.z));

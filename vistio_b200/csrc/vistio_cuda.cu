@@ -897,9 +897,11 @@ uint32_t launch_refinement(vistio_batch* b, cudaStream_t st) {
 }
 
 // The global solve: the sweeps, `refine` FP64 refinement sweeps, then the
-// residual sums and (plain step) the position update.
+// residual sums and, with them, the plain step's position update or the IPC
+// step's bounds.
 // With `reset` it clears those sums first (else the gather has).
-uint32_t launch_solve(vistio_batch* b, cudaStream_t st, int do_update, uint32_t refine, bool reset) {
+enum class After { kSums, kUpdate, kBounds };
+uint32_t launch_solve(vistio_batch* b, cudaStream_t st, After after, uint32_t refine, bool reset) {
   uint32_t n = 1 + reset;
   if (reset) launch_pdl(k_red_reset, (b->ninst + 127) / 128, 128, 0, st, b->dev, b->ninst);
   n += launch_sweeps(b, b->dev, st);
@@ -907,7 +909,8 @@ uint32_t launch_solve(vistio_batch* b, cudaStream_t st, int do_update, uint32_t 
     if (k) { launch_pdl(k_accum, b->n_vtx_chunks, kElemThreads, 0, st, b->dev); ++n; }
     n += launch_refinement(b, st);
   }
-  launch_pdl(k_update, b->n_vtx_chunks, 128, 0, st, b->dev, do_update, refine > 0);  // two vertices per thread
+  if (after == After::kBounds) launch_pdl(k_ipc_bounds, b->n_vtx_chunks, kElemThreads, 0, st, b->dev, refine > 0);
+  else launch_pdl(k_update, b->n_vtx_chunks, 128, 0, st, b->dev, after == After::kUpdate, refine > 0);  // two vertices per thread
   return n;
 }
 
@@ -929,7 +932,8 @@ void launch_bending(vistio_batch* b, cudaStream_t st) {
 // (7,700) 2508 -> 2544, 512 sheets 13.94 -> 14.60 ms.
 constexpr uint32_t kLocalChunks = 4 * 4 * 148;
 
-uint32_t launch_plain_iteration(vistio_batch* b, cudaStream_t st, int do_update, uint32_t refine) {
+// One PD iteration up to and with the pass over the vertices after its solve.
+uint32_t launch_iteration(vistio_batch* b, cudaStream_t st, bool ipc, uint32_t refine) {
   uint32_t n = 1;
   if (b->n_tri_chunks && b->n_hinge_chunks && b->n_tri_chunks + b->n_hinge_chunks <= kLocalChunks) {
     launch_pdl(k_local, b->n_tri_chunks + b->n_hinge_chunks, kElemThreads, 0, st, b->dev, b->n_tri_chunks);
@@ -939,7 +943,7 @@ uint32_t launch_plain_iteration(vistio_batch* b, cudaStream_t st, int do_update,
     if (b->n_hinge_chunks) { launch_bending(b, st); ++n; }
   }
   launch_pdl(k_gather, b->n_vtx_chunks, kElemThreads, 0, st, b->dev, refine > 0);
-  return n + launch_solve(b, st, do_update, refine, false);
+  return n + launch_solve(b, st, ipc ? After::kBounds : After::kUpdate, refine, false);
 }
 
 // One Augmented-Lagrangian pass of an IPC step. Returns the launches. It opens
@@ -954,9 +958,8 @@ uint32_t launch_al_pass(vistio_batch* b, bool self, cudaGraphConditionalHandle a
   for (uint32_t it = 0; it < b->cfg.max_iterations; ++it) {
     // With backtracking (alpha < 1) part of each sweep's error stays in x:
     // every solve is refined.
-    L += launch_plain_iteration(b, st, 0, b->refine) + 2;
-    if (self) launch_ccd_self(b->dev, b->self.view(), b->n_vtx_chunks, st);
-    else launch_pdl(k_ccd, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
+    L += launch_iteration(b, st, true, b->refine) + 1;
+    if (self) { launch_pdl(k_self_ccd, 6 * 148, kElemThreads, 0, st, b->dev, b->self.view()); ++L; }
     launch_pdl(k_ipc_update, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
   }
   if (self) L += launch_self_detect(b->dev, b->self.view(), b->n_vtx_chunks, b->n_tri_chunks, 1, st);
@@ -984,7 +987,7 @@ vistio_status capture(vistio_batch* b, bool ipc, bool self, cudaGraphExec_t* out
   if (!ipc) {
     // Each PD iteration recomputes its residual from x, so a sweep's error is
     // corrected by the next iteration; only the last solve is refined.
-    for (uint32_t it = 0; it < iters; ++it) L += launch_plain_iteration(b, st, 1, it + 1 == iters ? b->refine : 0);
+    for (uint32_t it = 0; it < iters; ++it) L += launch_iteration(b, st, false, it + 1 == iters ? b->refine : 0);
     launch_pdl(k_finalize, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
   } else {
     if (b->cfg.al_max_iterations) {
@@ -1797,7 +1800,7 @@ vistio_status vistio_batch_launch_phase(vistio_batch* b, int32_t phase) {
     case 1: launch_membrane(b, st); break;
     case 2: launch_bending(b, st); break;
     case 3: k_gather<<<b->n_vtx_chunks, kElemThreads, 0, st>>>(b->dev, b->refine > 0); break;
-    case 4: launch_solve(b, st, 0, 0, true); break;
+    case 4: launch_solve(b, st, After::kSums, 0, true); break;
     case 5: k_finalize<<<b->n_vtx_chunks, kElemThreads, 0, st>>>(b->dev); break;
     case 6:
       if (!b->refine) return fail(ctx, VISTIO_ERR_INVALID_CONFIG, "the batch has no refinement sweeps");
@@ -1923,7 +1926,7 @@ vistio_status vistio_sparse_solve(vistio_factor* f, const float* rhs, float* sol
   for (int pass = 0; pass < 3; ++pass) {
     for (uint32_t i = 0; i < n; ++i) y[f->f.iperm[i]] = make_float4(float(r[i]), 0.f, 0.f, 0.f);
     CU(cudaMemcpyAsync(b->Tm.p, y.data(), n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
-    launch_solve(b, ctx->stream, 0, 0, true);
+    launch_solve(b, ctx->stream, After::kSums, 0, true);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(y.data(), b->Y.p, n * sizeof(float4), cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
