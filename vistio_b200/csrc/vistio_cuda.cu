@@ -272,7 +272,7 @@ cudaError_t schedule(vistio_batch* b, uint32_t limit, cudaStream_t st) {
                                   : std::max(1u, uint32_t(per_item / chunks_in(S)));
         for (uint32_t t = 0; t < tiles; t += per) {
           items.push_back(SweepItem{dir == 0 ? S.f_off : S.b_off, S.vbase + S.first, S.vbase, S.ncols, S.nrows, S.rows_off,
-                                    S.inst, t, std::min(per, tiles - t), b->sn_pull[k], 0});
+                                    S.inst, t, std::min(per, tiles - t), b->sn_pull[k], b->sn_height[k] > 0});
           ++(warp ? L.nwarp : L.nblock);
         }
       }
