@@ -186,33 +186,38 @@ template <int DIR> struct Panel {
 
 // The children's updates at one of a supernode's columns or rows. The list is
 // read by prepare(), ahead of the wait; sum() reads the updates, in list order.
+// The sixteen-warp form reads four entries ahead (a single garment's sweep waits
+// for the rest of the list in every phase: 97x97 329 us per step, 334 with two,
+// 348 with one), the others two: four spill there (512 sheets 12.05 ms per step,
+// 11.91 with two, 24 sheets 1447 and 1429 us).
 // A warp item of a leaf reads no list (its lists are empty; 512 sheets 12.36 ->
 // 12.05 ms per step, 24 sheets 1493 -> 1448 us). Block items always do: few are
 // leaves, and the test cost single garments, which those bound, 1%.
-struct Pull {
-  uint32_t q, qe, slot[4];
+__host__ __device__ constexpr uint32_t list_ahead(uint32_t warps) { return warps == 16 ? 4 : 2; }
+template <uint32_t NP> struct Pull {
+  uint32_t q, qe, slot[NP];
   __device__ __forceinline__ void prepare(const BatchDev& B, uint32_t list) {
     q = __ldg(B.pull_ptr + list);
     qe = __ldg(B.pull_ptr + list + 1);
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) slot[i] = q + i < qe ? __ldg(B.pull + q + i) : 0u;
+    for (uint32_t i = 0; i < NP; ++i) slot[i] = q + i < qe ? __ldg(B.pull + q + i) : 0u;
   }
   __device__ __forceinline__ float4 sum(const BatchDev& B) const {
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i)
+    for (uint32_t i = 0; i < NP; ++i)
       if (q + i < qe) t = f4_add(t, B.U[slot[i]]);
 #pragma unroll 4
-    for (uint32_t e = q + 4; e < qe; ++e) t = f4_add(t, B.U[__ldg(B.pull + e)]);
+    for (uint32_t e = q + NP; e < qe; ++e) t = f4_add(t, B.U[__ldg(B.pull + e)]);
     return t;
   }
 };
 
 // One entry of v: what does not depend on other supernodes is read by prepare(),
 // ahead of the wait, the rest by get().
-template <int DIR, bool LEAVES> struct Entry {
+template <int DIR, uint32_t NP, bool LEAVES> struct Entry {
   uint32_t row;
-  Pull p;
+  Pull<NP> p;
   __device__ __forceinline__ void prepare(const BatchDev& B, const SweepItem& I, uint32_t c) {
     if (DIR == 0) {
       row = I.row0 + c;
@@ -229,9 +234,9 @@ template <int DIR, bool LEAVES> struct Entry {
 
 // One row of the product: begin() ahead of the wait, after() reads what the
 // result is combined with, put() writes it.
-template <int DIR, bool LEAVES> struct OutRow {
+template <int DIR, uint32_t NP, bool LEAVES> struct OutRow {
   uint32_t row;
-  Pull p;
+  Pull<NP> p;
   float4 with;
   __device__ __forceinline__ bool pulls(const SweepItem& I) const { return DIR == 0 && (!LEAVES || I.pulls) && row < I.nrows; }
   __device__ __forceinline__ void begin(const BatchDev& B, const SweepItem& I, uint32_t r) {
@@ -277,12 +282,12 @@ __device__ __forceinline__ void block_item(const BatchDev& B, const SweepItem& I
   };
   wrap();
   if (t < nt) M.issue(st, I.tile0 + t, ch);
-  OutRow<DIR, false> out;
+  OutRow<DIR, list_ahead(NW), false> out;
   if (warp < nt) out.begin(B, I, (I.tile0 + warp) * kTile + lane);
   float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t c0 = 0; c0 < M.cols; c0 += kVecCols) {
     const uint32_t nc = min(kVecCols, M.cols - c0);
-    Entry<DIR, false> e;
+    Entry<DIR, list_ahead(NW), false> e;
     if (tid < nc) e.prepare(B, I, c0 + tid);
     if (c0 == 0) {
       if (!wait()) {
@@ -345,12 +350,12 @@ __device__ __forceinline__ void block_item(const BatchDev& B, const SweepItem& I
 // One item of a supernode of at most kWarpCols columns by one warp: forward some
 // of its tiles, over its one or two chunks; backward one tile. v: kWarpCols
 // entries of the warp's own (backward a chunk at a time).
-template <int DIR, class Wait>
+template <int DIR, uint32_t NW, class Wait>
 __device__ __forceinline__ void warp_tiles(const BatchDev& B, const SweepItem& I, Stage& st, float4* v, Wait wait) {
   const Panel<DIR> M(B, I);
   const uint32_t lane = threadIdx.x & 31, all = (M.cols + kTile - 1) / kTile;
   M.issue(st, I.tile0, 0);
-  OutRow<DIR, true> out;
+  OutRow<DIR, list_ahead(NW), true> out;
   float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t t = 0; t < I.ntiles; ++t) {
     out.begin(B, I, (I.tile0 + t) * kTile + lane);
@@ -358,7 +363,7 @@ __device__ __forceinline__ void warp_tiles(const BatchDev& B, const SweepItem& I
       const uint32_t nc = M.chunk(ch);
       float4* vc = DIR == 0 ? v + ch * kTile : v;
       if (t == 0) {
-        Entry<DIR, true> e;
+        Entry<DIR, list_ahead(NW), true> e;
         if (lane < nc) e.prepare(B, I, ch * kTile + lane);
         if (ch == 0 && !wait()) {
           st.wait(B.status);  // the copy in flight lands before the block ends
@@ -412,7 +417,7 @@ k_level(BatchDev B, const SweepItem* __restrict__ items, uint32_t nblock, uint32
     return;
   }
   const SweepItem I = items[nblock + q];
-  warp_tiles<DIR>(B, I, st, v + warp * kWarpCols, [&]() {
+  warp_tiles<DIR, NW>(B, I, st, v + warp * kWarpCols, [&]() {
     pdl_begin();
     return !(B.prm->ipc && B.red[I.inst].al_done);
   });
