@@ -129,7 +129,8 @@ __device__ __forceinline__ float3 tri_centroid(const BatchDev& B, uint32_t tri) 
 
 // The bounds of each garment's centroids, one block per 256 triangles (bounds
 // starts at all ones for the minima and zero for the maxima). With k_self_keys,
-// against one block per garment: folded ribbon of 32,000 triangles 57 -> 8 us.
+// against one block per garment: folded ribbon of 32,000 triangles 57 -> 12 us (7
+// and 5).
 __global__ void __launch_bounds__(256) k_self_bounds(BatchDev B, SelfContactView S) {
   pdl_begin();
   const int4 ch = B.tri_chunks[blockIdx.x];
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const uint64_t* __restrict__
 // Leaf boxes (bvh.rs:29-43, inflated by the margin) and the levels above them
 // that 256 leaves reach, one block per 256 leaves; then, one block per garment,
 // the few levels above those. Against one block per garment for all levels:
-// folded ribbon of 32,000 triangles 91 -> 10 us, 64 drapes 70 -> 30 us.
+// folded ribbon of 32,000 triangles 91 -> 12 us (7 and 5), 64 drapes 70 -> 29 us.
 __device__ __forceinline__ float4 min4(float4 a, float4 b) { return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.f); }
 __device__ __forceinline__ float4 max4(float4 a, float4 b) { return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f); }
 constexpr uint32_t kLeafLevels = 8;  // levels above the leaves that one block of 256 leaves builds

@@ -31,10 +31,11 @@
 // for the backward one): the same bytes are read either way.
 //
 // Against inv(L_kk) and L_Rk over a tree of 9 to 11 levels, swept by one
-// persistent dependency-driven launch (time of a whole plain step of 10 solves,
-// B200): sheet 20x20 720 -> 396 us with the state read back, 97x97 with a
-// refinement 3956 -> 1425 us for two steps, 24 sheets of sides 17 to 151
-// 3.83 -> 2.11 ms, 512 sheets of sides 23 to 121 15.4 -> 14.0 ms.
+// persistent dependency-driven launch (time of whole plain steps of 10 solves,
+// B200): sheet 20x20 721 -> 306 us with the state read back, 97x97 with a
+// refinement 3958 -> 946 us for two steps, 24 sheets of sides 17 to 151
+// 3.80 -> 1.52 ms, 512 sheets of sides 23 to 121 15.29 -> 12.15 ms. By phase the last
+// reads 2.6 to 4.9 TB/s (2.62 GB in 711 us), the small phases at the top less.
 #pragma once
 #include "pd_kernels.cuh"
 

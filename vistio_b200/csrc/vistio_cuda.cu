@@ -973,8 +973,9 @@ uint32_t launch_al_pass(vistio_batch* b, bool self, cudaGraphConditionalHandle a
 // a conditional (while) node: a pass that every garment is done with is not
 // launched at all. As al_max_iterations copies of the pass in one graph, each
 // whose garments were done still cost its 150 to 250 launches that return at
-// once: drape 64x64 (4 of 10 passes needed in two steps) 4290 us, folded ribbon
-// 40x400 (2 of 10) 8970 us, and five times the nodes to instantiate.
+// once: drape 64x64 (4 of 10 passes needed in two steps) 4290 -> 3074 us, folded
+// ribbon 40x400 (2 of 10) 8970 -> 5460 us, 64 drapes 24.0 -> 21.2 ms (each against
+// the same kernels without the node), and a fifth of the nodes to instantiate.
 vistio_status capture(vistio_batch* b, bool ipc, bool self, cudaGraphExec_t* out, uint32_t* nlaunch) {
   vistio_ctx* ctx = b->ctx;
   cudaStream_t st = ctx->stream;
