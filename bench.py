@@ -860,7 +860,10 @@ def main():
         os.path.join(ROOT, "MEASURED_PEAKS.json")) else None
     peak = peaks["hbm_gbs"] if peaks else 6650.0  # fallback: an earlier copy-bandwidth measurement
     achieved = alg[dom] / (kern_ms[dom] * 1e-3) / 1e9
-    solve_kernels = "k_red_reset + k_level (one launch per phase of the sweeps) + k_update"
+    solve_kernels = {"dataflow": "k_red_reset + k_sweep + k_update",
+                     "grouped": "k_red_reset + k_gsweep<0> + k_sweep + k_gsweep<1> + k_update",
+                     "levels": "k_red_reset + k_subtree<0> + k_level<0> x L + k_level<1> x L + k_subtree<1> + k_update"
+                     }[batch.sweep_mode()[0]]
     roofline = {"bound": "hbm", "kernel": {"solve": solve_kernels, "membrane": "k_tri", "bending": "k_hinge",
                                           "gather": "k_gather"}[dom],
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -276,26 +276,28 @@ vistio_status vistio_batch_info(const vistio_batch* b, uint32_t* n_instances, ui
                                 uint64_t* device_bytes);
 /* Autotuner of the sweeps (no counterpart in the reference). Two things are
  * chosen by timing this batch's forward and backward sweeps:
- * - the sweep kind, an order of the work; every kind is one kernel launch per
- *   phase of independent supernodes and gives the same results, bit for bit:
- *   0 = phases by height above the leaves of the supernodal trees, heaviest
- *   supernodes first; 1 = phases by depth below the roots, so that what a
- *   supernode waits for is as late as it can be; 2 (batches with garment
- *   groups: at least 8 garments of one mesh topology) = as 0 with the groups'
- *   supernodes last and the same supernode of a topology's garments side by
- *   side;
- * - which supernodes a single warp takes and which a whole block, by a limit
- *   on s (s + m): 0, 1024, 2048, 4096, 6144, 12288 and 2^30.
+ * - the sweep kind: 0 = one kernel launch per level of the supernodal trees;
+ *   1 = one dependency-driven launch for both directions, in which each
+ *   supernode waits only for its own children (forward) or parent (backward);
+ *   2 (batches with garment groups: at least 8 garments of one mesh topology)
+ *   = the bottom of the groups' trees swept one lane per garment, before and
+ *   after kind 1 sweeps the rest;
+ * - which of the top-level supernodes that a single warp takes (at most 32
+ *   columns, s (s + m) at most 6144) share a work unit of kinds 1 and 2, by a
+ *   limit on s (s + m): 0, 1024, 2048, 4096, 6144, 12288 and 2^30. One above
+ *   the limit has a unit for itself; limits from 6144 on are the same.
+ * Every kind and limit gives the same results, bit for bit.
  * candidate_ms (21 entries, may be NULL) receives the time of each limit for
  * kind 0 (entries 0-6) and kind 1 (entries 7-13); entries 14-20 time kind 2 at
  * kind 1's fastest limit with the group limits 0, 64, 128, 256, 512, 1024 and
- * 6144 (the largest s (s + m) of a supernode above the leaves that is ordered
- * that way; -1 without garment groups or above that warp-item limit). The fastest candidate is kept (*chosen_limit; the
+ * 6144 (the largest s (s + m) of a supernode above the bottom subtrees that
+ * the groups sweep one lane per garment; -1 without garment groups or above
+ * that warp-item limit). The fastest candidate is kept (*chosen_limit; the
  * kind from vistio_batch_get_sweep_mode, the group limit from
  * vistio_batch_get_group_limit). Without tuning: kind 2 if the batch has
- * garment groups, else kind 1, with the limits 6144. The chosen schedule is
- * then timed with the compiled forms of the sweep kernel
- * (vistio_batch_get_sweep_blocks). Captured step graphs are
+ * garment groups, else kind 1, with the limits 6144. For kinds 1 and 2 the
+ * chosen schedule is then timed with both compiled forms of the dependency-
+ * driven kernel (vistio_batch_get_sweep_blocks). Captured step graphs are
  * rebuilt on the next step. Synchronises the batch's stream. */
 vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* candidate_ms);
 /* Autotunes the shapes of the local steps on this batch (no reference
@@ -330,13 +332,14 @@ vistio_status vistio_batch_set_warp_limit(vistio_batch* b, uint32_t limit);
 vistio_status vistio_batch_set_sweep_mode(vistio_batch* b, uint32_t mode);
 /* The sweep kind and warp-item limit in use. */
 vistio_status vistio_batch_get_sweep_mode(const vistio_batch* b, uint32_t* mode, uint32_t* warp_limit);
-/* The sweep kernel is compiled in three forms, named by resident blocks per
- * SM: 5 (six-warp blocks), 4 (eight warps) and 2 (sixteen warps); no reference
- * counterpart. vistio_batch_tune times the three with the schedule it chose
- * and keeps the fastest; without tuning, 2 for a batch of at most 8 garments,
- * else 4. All give the same results, bit for bit. get: the form in use and, in
- * tuned_ms (3 entries, may be NULL), the tuner's times of the forms 5, 4 and 2
- * (-1 before tuning). */
+/* The dependency-driven sweep kernel (kinds 1 and 2) is compiled in three
+ * forms, named by resident blocks per SM: 5 and 4 (eight-warp blocks, 48 and
+ * 64 registers per thread) and 2 (sixteen-warp blocks, whose units hold twice
+ * as many items); no reference counterpart. vistio_batch_tune times the three
+ * with the schedule it chose and keeps the fastest; without tuning, 2 for a
+ * batch of at most 8 garments, else 4. All give the same results, bit for
+ * bit. get: the form in use and, in tuned_ms (3 entries, may be NULL), the
+ * tuner's times of the forms 5, 4 and 2 (-1 before tuning or for kind 0). */
 vistio_status vistio_batch_set_sweep_blocks(vistio_batch* b, uint32_t blocks_per_sm);
 vistio_status vistio_batch_get_sweep_blocks(const vistio_batch* b, uint32_t* blocks_per_sm, float* tuned_ms);
 /* The device factorization done when the batch was created (the garments
@@ -383,7 +386,10 @@ typedef struct vistio_server_config {
    * is overridden); 1: each request's own setting (0 = its cohort factorizes
    * on the GPU when it starts, on the thread that calls vistio_server_tick). */
   uint32_t gpu_factorization;
-  /* Sweep kind of every cohort (vistio_batch_set_sweep_mode): 0 or 1. */
+  /* Sweep kind of every cohort (vistio_batch_set_sweep_mode): 0 = one launch
+   * per level, 1 = dependency-driven. Cohorts run side by side on their own
+   * streams, and the dependency-driven sweeps keep blocks resident that wait
+   * for one another, so 0 suits a busy server. */
   uint32_t sweep_mode;
   /* Admission window: while any cohort is running, ready requests of one step
    * configuration wait up to this long (from the first one's readiness) for

@@ -476,8 +476,8 @@ class Batch:
                              "bending": {"1": float(lms[2]), "2": float(lms[3])}}}
 
     def set_group_limit(self, limit: int):
-        """Largest s (s + m) of a supernode above the leaves that the sweep kind
-        "grouped" orders by topology."""
+        """Largest s (s + m) of a supernode above the bottom subtrees that the
+        garment groups sweep one lane per garment (sweep kind "grouped")."""
         L.check(L.lib().vistio_batch_set_group_limit(self.h, int(limit)), self.ctx.h)
 
     def group_limit(self) -> int:
@@ -497,19 +497,21 @@ class Batch:
         L.check(L.lib().vistio_batch_set_self_ccd_dedup(self.h, 1 if on else 0), self.ctx.h)
 
     def set_warp_limit(self, limit: int):
+        """Largest s (s + m) of the supernodes of one warp that share a work unit
+        of the dependency-driven sweeps; bit-identical results."""
         L.check(L.lib().vistio_batch_set_warp_limit(self.h, int(limit)), self.ctx.h)
 
     def set_sweep_mode(self, mode: str):
-        """Order of the sweeps' work (bit-identical results). "levels": phases
-        by height above the leaves of the supernodal trees; "dataflow": by
-        depth below the roots; "grouped" (batches with garment groups: 8 or
-        more garments of one mesh topology): by height, the same supernode of a
-        topology's garments side by side."""
+        """"levels": one launch per level; "dataflow": one dependency-driven
+        launch for both directions; "grouped" (batches with garment groups:
+        8 or more garments of one mesh topology): the groups' tree bottoms
+        one lane per garment, the rest dependency-driven."""
         L.check(L.lib().vistio_batch_set_sweep_mode(self.h, self.SWEEP_MODES.index(mode)), self.ctx.h)
 
     def set_sweep_blocks(self, blocks_per_sm: int):
-        """Compiled form of the sweep kernel, by resident blocks per SM: 5
-        (six-warp blocks), 4 (eight) or 2 (sixteen); bit-identical results."""
+        """Compiled form of the dependency-driven sweep kernel, by resident
+        blocks per SM: 5 or 4 (eight-warp blocks) or 2 (sixteen-warp blocks);
+        bit-identical results."""
         L.check(L.lib().vistio_batch_set_sweep_blocks(self.h, int(blocks_per_sm)), self.ctx.h)
 
     def sweep_blocks(self) -> tuple:

@@ -205,15 +205,14 @@ __global__ void __launch_bounds__(256) k_detect(BatchDev B, int mode) {
 }
 
 // After the sweeps of an IPC iteration, per vertex in one pass: the residual sums
-// (pd_solver.rs:403-421), d in vertex order into T (the sweeps are done with
-// their right-hand side; the self-contact CCD and the update read it there), the
-// CCD step bound of the colliders (ground_plane.rs:112-134, sphere.rs:178-224,
-// cylinder.rs:201-262, box_collider.rs:203-251) and the backtracking sum grad . d
-// over free vertices (pd_solver.rs:915-925). add_w folds the last refinement
-// correction into d. As two kernels (sums, then bounds) a drape of 64x64 took
-// 2.35 ms per step, now 2.26. The sums leave the block by one atomic each: all
-// blocks of a garment add to one address, and an atomic per warp cost a ribbon of
-// 40x400 3.70 -> 3.80 ms.
+// (pd_solver.rs:403-421), d in vertex order into T (the self-contact CCD and the
+// update read it there), the CCD step bound of the colliders
+// (ground_plane.rs:112-134, sphere.rs:178-224, cylinder.rs:201-262,
+// box_collider.rs:203-251) and the backtracking sum grad . d over free vertices
+// (pd_solver.rs:915-925). add_w folds the last refinement correction into d. As
+// two kernels (sums, then bounds) two steps of a drape of 64x64 took 0.09 ms more.
+// The sums leave the block by one atomic each: all blocks of a garment add to one
+// address, and an atomic per warp added 0.1 ms to two steps of a ribbon of 40x400.
 __global__ void __launch_bounds__(256) k_ipc_bounds(BatchDev B, int add_w) {
   pdl_begin();
   int4 ch = B.vtx_chunks[blockIdx.x];

@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <iterator>
 #include <limits>
 #include <condition_variable>
 #include <memory>
@@ -528,90 +527,61 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
     }
     sns.swap(out);
   }
-  // Merge the supernodal tree into few levels. A sweep's time on a small batch
-  // is the number of dependent levels, not the factor's bytes: each level costs
-  // a signal and a few round trips through L2 whatever its size. So every
-  // subtree of at most the first of kMergeCols' limits becomes one supernode,
-  // then every subtree of what remains of at most the second, and so on; the
-  // last limit repeats until nothing remains. Rows below a merged supernode are
-  // those of its topmost part (the parts below it only reach into the merged
-  // columns and those rows).
-  uint32_t nfine = uint32_t(sns.size());
-  std::vector<uint32_t> fine_of(n), fine_parent(nfine, UINT32_MAX), head(nfine, UINT32_MAX);
-  for (uint32_t k = 0; k < nfine; ++k)
-    for (uint32_t j = sns[k].f; j < sns[k].f + sns[k].s; ++j) fine_of[j] = k;
-  for (uint32_t k = 0; k < nfine; ++k)
-    if (!sns[k].below.empty()) fine_parent[k] = fine_of[sns[k].below[0]];
-  const MergeCols* merge = kMergeCols;
-  while (n > merge->max_n) ++merge;
-  for (uint32_t l = 0, left = nfine; left; ++l) {
-    const uint64_t limit = merge->cols[std::min<size_t>(l, std::size(merge->cols) - 1)];
-    std::vector<uint64_t> cols(nfine, 0);
-    for (uint32_t k = 0; k < nfine; ++k) {  // children precede parents
-      if (head[k] != UINT32_MAX) continue;
-      cols[k] += sns[k].s;
-      if (fine_parent[k] != UINT32_MAX) cols[fine_parent[k]] += cols[k];
-    }
-    std::vector<uint32_t> now(nfine, UINT32_MAX);
-    for (uint32_t k = nfine; k-- > 0;) {
-      if (head[k] != UINT32_MAX) continue;
-      const uint32_t p = fine_parent[k];
-      if (p != UINT32_MAX && now[p] != UINT32_MAX) now[k] = now[p];
-      else if (cols[k] <= limit) now[k] = k;
-    }
-    for (uint32_t k = 0; k < nfine; ++k)
-      if (now[k] != UINT32_MAX) { head[k] = now[k]; --left; }
-  }
-  // The merged supernodes in the order of their topmost parts (children first),
-  // their columns in elimination order and made contiguous: another
-  // topological order of the elimination tree, so the same fill.
-  std::vector<std::vector<uint32_t>> parts(nfine);
-  for (uint32_t k = 0; k < nfine; ++k) parts[head[k]].push_back(k);
-  std::vector<uint32_t> newpos(n), heads;
-  {
-    uint32_t at = 0;
-    for (uint32_t h = 0; h < nfine; ++h) {
-      if (parts[h].empty()) continue;
-      heads.push_back(h);
-      for (uint32_t k : parts[h])
-        for (uint32_t j = sns[k].f; j < sns[k].f + sns[k].s; ++j) newpos[j] = at++;
-    }
-    std::vector<uint32_t> perm2(n);
-    for (uint32_t j = 0; j < n; ++j) perm2[newpos[j]] = f.perm[j];
-    f.perm.swap(perm2);
-    for (uint32_t j = 0; j < n; ++j) f.iperm[f.perm[j]] = j;
-  }
-  uint32_t nsn = uint32_t(heads.size());
+  // Owner map, parents, levels.
+  uint32_t nsn = uint32_t(sns.size());
   f.row_sn.assign(n, 0);
+  for (uint32_t k = 0; k < nsn; ++k)
+    for (uint32_t j = sns[k].f; j < sns[k].f + sns[k].s; ++j) f.row_sn[j] = k;
   f.sn.resize(nsn);
   uint64_t off = 0;
-  for (uint32_t k = 0, first = 0; k < nsn; ++k) {
+  for (uint32_t k = 0; k < nsn; ++k) {
     Supernode& S = f.sn[k];
-    const SN& top = sns[heads[k]];
-    S.first = first;
-    S.ncols = 0;
-    for (uint32_t q : parts[heads[k]]) S.ncols += sns[q].s;
-    first += S.ncols;
-    for (uint32_t j = S.first; j < first; ++j) f.row_sn[j] = k;
-    S.nrows = uint32_t(top.below.size());
+    S.first = sns[k].f;
+    S.ncols = sns[k].s;
+    S.nrows = uint32_t(sns[k].below.size());
     S.rows_off = uint32_t(f.rows.size());
-    for (uint32_t r : top.below) f.rows.push_back(newpos[r]);
-    std::sort(f.rows.begin() + S.rows_off, f.rows.end());
+    f.rows.insert(f.rows.end(), sns[k].below.begin(), sns[k].below.end());
     S.panel_off = off;
     off += uint64_t(S.nrows) * S.ncols;
     S.diag_off = off;
     off += uint64_t(S.ncols) * S.ncols;
+    S.parent = S.nrows ? f.row_sn[sns[k].below[0]] : UINT32_MAX;
+    S.level = 0;
   }
-  // Parents, and levels: the leaves are listed apart (kBottomLevel), and a
-  // supernode above them has one level more than its highest child.
+  // Bottom subtrees whose packed data fits kSubtreeFloats and whose columns
+  // number at most kSubtreeCols are swept whole by one warp; the supernodes
+  // above them are swept level by level, a top
+  // supernode's level being one more than its highest top child (children
+  // that are bottom subtrees count as below level 0).
   {
-    std::vector<int> lvl(nsn, -1);
+    std::vector<uint64_t> sub(nsn, 0), cols(nsn, 0);
+    std::vector<uint32_t> cnt_sub(nsn, 1);
+    for (uint32_t k = 0; k < nsn; ++k) {  // children precede parents (postorder)
+      sub[k] += sn_floats(f.sn[k].ncols, f.sn[k].nrows);
+      cols[k] += f.sn[k].ncols;
+      uint32_t p = f.sn[k].parent;
+      if (p != UINT32_MAX) { sub[p] += sub[k]; cols[p] += cols[k]; cnt_sub[p] += cnt_sub[k]; }
+    }
+    std::vector<char> bottom(nsn, 0);
+    for (int k = int(nsn) - 1; k >= 0; --k) {  // parents first
+      uint32_t p = f.sn[k].parent;
+      bool fits = sub[k] <= kSubtreeFloats && cols[k] <= kSubtreeCols;
+      if (p != UINT32_MAX && bottom[p]) bottom[k] = 1;
+      else if (fits) {
+        bottom[k] = 1;
+        f.sub_first.push_back(uint32_t(k) + 1 - cnt_sub[k]);
+        f.sub_last.push_back(uint32_t(k));
+      }
+    }
+    std::reverse(f.sub_first.begin(), f.sub_first.end());
+    std::reverse(f.sub_last.begin(), f.sub_last.end());
+    std::vector<int> top_lvl(nsn, -1);
     for (uint32_t k = 0; k < nsn; ++k) {
-      Supernode& S = f.sn[k];
-      S.parent = S.nrows ? f.row_sn[f.rows[S.rows_off]] : UINT32_MAX;
-      S.level = lvl[k] < 0 ? kBottomLevel : uint32_t(lvl[k]);
-      if (lvl[k] < 0) { f.sub_first.push_back(k); f.sub_last.push_back(k); }
-      if (S.parent != UINT32_MAX) lvl[S.parent] = std::max(lvl[S.parent], lvl[k] + 1);
+      if (bottom[k]) { f.sn[k].level = kBottomLevel; continue; }
+      if (top_lvl[k] < 0) top_lvl[k] = 0;
+      f.sn[k].level = uint32_t(top_lvl[k]);
+      uint32_t p = f.sn[k].parent;
+      if (p != UINT32_MAX) top_lvl[p] = std::max(top_lvl[p], top_lvl[k] + 1);
     }
   }
   f.nnz_stored = off;
@@ -619,8 +589,6 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
   // Scatter the simplicial columns into panels and diagonal blocks.
   std::vector<int> pos(n, -1);
   std::vector<double> Lkk;
-  std::vector<uint32_t> oldpos(n);
-  for (uint32_t j = 0; j < n; ++j) oldpos[newpos[j]] = j;
   for (uint32_t k = 0; k < nsn && numeric; ++k) {
     Supernode& S = f.sn[k];
     const uint32_t* R = f.rows.data() + S.rows_off;
@@ -628,9 +596,9 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
     uint32_t s = S.ncols;
     Lkk.assign(size_t(s) * s, 0.0);
     for (uint32_t c = 0; c < s; ++c) {
-      uint32_t j = oldpos[S.first + c];
+      uint32_t j = S.first + c;
       for (uint64_t q = Lp[j]; q < Lp[j + 1]; ++q) {
-        uint32_t i = newpos[Li[q]];
+        uint32_t i = Li[q];
         if (i < S.first + s) Lkk[size_t(c) * s + (i - S.first)] = Lx[q];  // column-major
         else {
           int pr = pos[i];
@@ -640,18 +608,14 @@ std::string factorize_csr(uint32_t n, const uint32_t* row_ptr, const uint32_t* c
       }
     }
     for (uint32_t r = 0; r < S.nrows; ++r) pos[R[r]] = -1;
-    // inv(L_kk) by forward substitution on the identity, column by column
-    // (both column-major: the inner loop runs down contiguous columns).
+    // inv(L_kk) by forward substitution on the identity (column-major).
     double* Inv = f.vals.data() + S.diag_off;
     for (uint32_t c = 0; c < s; ++c) {
-      double* x = Inv + size_t(c) * s;
-      std::fill(x, x + s, 0.0);
-      x[c] = 1.0;
-      for (uint32_t m = c; m < s; ++m) {
-        const double* col = Lkk.data() + size_t(m) * s;
-        const double v = x[m] / col[m];
-        x[m] = v;
-        for (uint32_t i = m + 1; i < s; ++i) x[i] -= col[i] * v;
+      // column c of inverse: solve L y = e_c
+      for (uint32_t i = 0; i < s; ++i) {
+        double v = (i == c) ? 1.0 : 0.0;
+        for (uint32_t m = c; m < i; ++m) v -= Lkk[size_t(m) * s + i] * Inv[size_t(c) * s + m];
+        Inv[size_t(c) * s + i] = (i < c) ? 0.0 : v / Lkk[size_t(i) * s + i];
       }
     }
   }

@@ -28,36 +28,35 @@ struct SetupParams {
   bool numeric = true;            // false: symbolic factorization only (the numbers on the GPU)
 };
 
-// Largest fundamental supernode (columns) before the tree is merged.
+// Largest supernode (columns); the GPU sweeps size their shared-memory vectors for it.
 constexpr uint32_t kMaxSupernodeCols = 256;
-// The supernodal tree is merged into few levels: subtrees of at most cols[0]
-// columns become one supernode each, then subtrees of the rest of at most
-// cols[1] columns, and so on (the last limit repeats). Wide limits give fewer
-// levels, which bound a few garments, and more factor bytes, which bound many.
-// The garment's size alone decides (its result must not depend on its batch);
-// plain steps of 10 iterations (us, one garment / 16 / 128 of it) with the three
-// rows below, the one taken marked:
-//   side  45    *211 /  332 / 1421    266 /  341 / 1394    322 /  399 / 1420
-//         64    *271 /  541 / 2618    280 /  554 / 2619    348 /  519 / 2491
-//         97     292 / 1070 / 5893   *332 / 1078 / 5546    401 / 1096 / 5374
-//        121     346 / 1821 / 10721   356 / 1613 / 8844   *414 / 1600 / 8094
-//        150     420 / 2604 / 15820   412 / 2504 / 14505  *443 / 2353 / 12526
-struct MergeCols {
-  uint32_t max_n;    // vertices up to which the row is taken
-  uint32_t cols[5];
-};
-constexpr MergeCols kMergeCols[] = {{5000, {128, 512, 1024, 1024, 1024}},
-                                    {11000, {48, 160, 512, 1024, 1024}},
-                                    {0xffffffffu, {32, 80, 200, 500, 1024}}};
-constexpr uint32_t kBottomLevel = 0xffffffffu;  // level of a leaf of the merged tree
-// Floats of one supernode's two panels as packed for the GPU (see SnDev):
-// forward, s columns of m + s rows; backward, m columns of s rows; rows padded
-// to 8.
-inline uint64_t pad8(uint64_t n) { return (n + 7) & ~uint64_t(7); }
-inline uint64_t sn_floats(uint32_t s, uint32_t m) { return uint64_t(s) * pad8(m + s) + uint64_t(m) * pad8(s); }
+// Bottom subtrees of the supernodal elimination tree whose factor data (in
+// floats, as packed for the GPU: sn_floats per supernode) fits this budget
+// are swept as one unit by one warp.
+constexpr uint32_t kSubtreeFloats = 1024;
+// ... and whose columns (contiguous in postorder) number at most this: the
+// warp keeps the subtree's slice of the vector in shared memory.
+constexpr uint32_t kSubtreeCols = 32;
+constexpr uint32_t kBottomLevel = 0xffffffffu;
+#if defined(__CUDACC__)
+#define VISTIO_HD __host__ __device__
+#else
+#define VISTIO_HD
+#endif
+// Leading dimension of a supernode's diagonal block (column-major) and panel
+// (row-major) as packed for the GPU: s rounded up to an odd number, so that
+// 32 lanes reading one column of 32 consecutive panel rows, or one row of 32
+// consecutive diagonal-block columns, hit 32 different shared-memory banks.
+VISTIO_HD constexpr uint32_t sn_ld(uint32_t s) { return s | 1u; }
+// Floats of one supernode's packed region: inv(L_kk) (s columns of sn_ld(s)),
+// then the panel (m rows of sn_ld(s)) followed by its m row indices, each
+// part padded to 4 floats.
+inline uint64_t sn_floats(uint32_t s, uint32_t m) {
+  return ((uint64_t(s) * sn_ld(s) + 3) & ~3ull) + ((uint64_t(m) * sn_ld(s) + m + 3) & ~3ull);
+}
 
-// Supernodal factor of P A P^T = L L^T over the merged supernodes. Columns are
-// in the permuted (elimination) order.
+// Supernodal factor of P A P^T = L L^T in the layout the GPU sweeps read.
+// Columns are in the permuted (elimination) order.
 struct Supernode {
   uint32_t first;     // first column
   uint32_t ncols;     // s
@@ -66,7 +65,7 @@ struct Supernode {
   uint64_t panel_off; // offset of the |R| x s row-major panel in Factor::vals
   uint64_t diag_off;  // offset of inv(L_kk), s x s column-major, in Factor::vals
   uint32_t parent;    // parent supernode, or UINT32_MAX for a root
-  uint32_t level;     // sweep level above the leaves of the tree (kBottomLevel for a leaf)
+  uint32_t level;     // sweep level above the bottom subtrees (kBottomLevel inside one)
 };
 
 struct Factor {
@@ -83,7 +82,7 @@ struct Factor {
   std::vector<uint32_t> level_rows; // rows (columns) of the level's supernodes, grouped by supernode
   std::vector<uint32_t> level_sn_ptr; // nlevels+1 offsets into level_sn
   std::vector<uint32_t> level_sn;     // supernodes of each level, largest first
-  // The leaves of the tree, as supernode ranges [first, last] of one each.
+  // Bottom subtrees: supernode ranges [first, last] in postorder (last = root).
   std::vector<uint32_t> sub_first, sub_last;
   // Forward-sweep pull lists: for each row r, the (supernode, panel row) pairs
   // of the descendants whose panels hold row r.

@@ -21,9 +21,10 @@
 #include "factor_kernels.cuh"
 #include "self_contact.cuh"
 #include "setup.h"
-#include "solve_kernels.cuh"
 
 using namespace vistio;
+static_assert(kSubtreeFloats <= kWarpFloats, "a bottom subtree must fit one warp buffer");
+static_assert(kSubtreeCols <= kWarpVec, "a bottom subtree's vector slice must fit one warp's vector slots");
 
 struct vistio_ctx {
   int device = 0;
@@ -34,6 +35,8 @@ struct vistio_ctx {
   std::mutex mu;
   int refs = 0;
   bool closed = false;
+  uint32_t sweep_blocks[3] = {0, 0, 0};  // resident k_sweep blocks on this device: the five- and four-block eight-warp forms, the sixteen-warp form
+  uint32_t gsweep_blocks = 0;  // resident k_gsweep blocks
 };
 
 namespace {
@@ -78,7 +81,8 @@ struct vistio_solver {
 namespace {
 
 constexpr int kElemThreads = 256;
-constexpr uint32_t kNoParent = 0xffffffffu;  // of a root supernode
+constexpr int kSolveThreads = 32 * kSolveWarps;
+constexpr uint32_t kWideSmem = kWideWarps * (kWarpFloats * 4 + 3 * kWarpVec * 16);
 
 thread_local std::string g_tls_error;
 
@@ -143,8 +147,10 @@ struct vistio_batch {
   DevBuf<uint4> tri_idx, hinge_idx;
   DevBuf<float4> tri_dm, hinge_st;
   DevBuf<float2> hinge_wr;
-  DevBuf<uint32_t> vtri_ptr, vtri, vhinge_ptr, vhinge, perm_local, rows, pull_ptr, pull, status;
-  uint32_t factor_launches = 0;  // launches of the device factorization
+  DevBuf<uint32_t> vtri_ptr, vtri, vhinge_ptr, vhinge, perm_local, rows, lvl_items, fwd_ptr, fwd, status;
+  DevBuf<uint2> sub_items;
+  uint32_t n_sub = 0;
+  uint32_t factor_launches = 0;  // k_front launches of the device factorization
   float factor_ms = 0.f;         // their device time
   // FP64 refinement: permuted f64 CSR of A, kept right-hand side, correction
   DevBuf<uint32_t> a_ptr, a_col;
@@ -152,36 +158,58 @@ struct vistio_batch {
   DevBuf<float4> R0, W;
   uint32_t refine = 0;       // refinement sweeps per refined solve
   BatchDev dev_w{};          // dev with Y = W: the sweeps of a refinement
-  // the sweeps' schedule (see schedule()): their phases in launch order
-  struct Phase { int dir; uint32_t off, nblock, nwarp; };
-  std::vector<Phase> phases;
+  // batch levels of the sweeps: offset into lvl_items, block items, warp items
+  std::vector<uint32_t> lvl_off, lvl_nb, lvl_nw;
+  std::vector<std::pair<uint32_t, uint32_t>> top;  // (level, supernode) of every top-level supernode
   std::vector<SnDev> sn_host;                       // supernode table, for re-scheduling
-  std::vector<uint32_t> sn_height, sn_depth;        // levels below / above each supernode in its tree
-  std::vector<uint32_t> sn_parent;                  // global ids, kNoParent at a root
-  std::vector<uint32_t> sn_pull;                    // first pull list of each supernode
-  // per global supernode: (structure class << 32) | local id. Schedules take
-  // equal keys side by side (the same supernode of garments that share a
-  // topology: equal work, shared row indices).
+  // per global supernode: (structure class << 32) | local id. Work units of
+  // the per-garment sweeps take equal keys side by side (the same supernode
+  // of garments that share a topology: equal work for the block's warps).
   std::vector<uint64_t> sn_key;
-  std::vector<uint8_t> sn_in_group;                 // of a garment in a group
-  uint32_t warp_limit = kWarpItemLimit;             // s (s + m) limit of a warp item
+  uint32_t warp_limit = kWarpItemLimit;             // s (s + m) limit of the warp items that share a unit
   uint32_t tri_per = 2, hinge_per = 1;              // elements per thread of k_tri / k_hinge (autotuned)
   uint32_t self_ccd_dedup = 1;                      // self CCD over each vertex-triangle test once
   float tuned_ms = 0.f;                             // sweep time of the tuned schedule (0: not tuned)
   float occ_ms[3] = {-1.f, -1.f, -1.f};  // the autotuner's times of the three forms (ms per solve)
-  // k_level's compiled form, by blocks per SM: 5 or 4 (eight warps), 2
-  // (sixteen warps); the autotuner's choice
+  // k_sweep's compiled form, by blocks per SM: 5 or 4 (eight warps), 2
+  // (sixteen warps, units of 2 kUnitItems items); the autotuner's choice
   uint32_t sweep_occ = 4;
-  // order of the sweeps' work (the results do not depend on it): supernodes in
-  // phases by their height above the leaves, heaviest first (0); by their depth
-  // below the root (1); as 0 with the groups' supernodes up to group_limit side
-  // by side, the same supernode of every garment of a topology (2)
+  uint32_t unit_items = kUnitItems;  // items per subtree or warp-supernode unit of the schedule
+  // sweeps: 0 = one launch per level (k_level), 1 = dependency-driven (k_sweep),
+  // 2 = garment groups' tree bottoms by k_gsweep, the rest by k_sweep
   uint32_t sweep_mode = 1;
-  uint32_t group_limit = kWarpItemLimit;            // largest s (s + m) of those above the leaves
-  uint32_t n_groups = 0;
-  DevBuf<SweepItem> items;
+  std::vector<uint2> units_host;                    // k_sweep work units in forward order
+  uint32_t n_units = 0, n_units_fwd = 0;
+  std::vector<uint2> units_fwd_host;                // k_sweep forward units: top supernodes deepest first
+  std::vector<uint32_t> items_fwd_host;             // their warp supernodes, bundled by depth
+  std::vector<uint32_t> sn_depth;                   // ancestors of each supernode in its tree
+  DevBuf<uint2> df_units_fwd;
+  DevBuf<uint32_t> df_items_fwd;
+  DevBuf<uint2> df_units;
+  DevBuf<uint32_t> df_parent, df_nkids, df_kid_ptr, df_kids, df_cnt, df_flag, df_queue;
   DevBuf<SnDev> sn;
   DevBuf<float4> U;
+  // garment groups (k_gsweep, sweep mode 2): the bottom of the trees of
+  // garments that share a symbolic structure, swept one lane per garment
+  uint32_t n_groups = 0, n_gitems_fwd = 0, n_gitems_bwd = 0, n_gpack = 0, n_sub_plain = 0;
+  std::vector<uint8_t> sn_grouped;  // per global supernode: swept by k_gsweep in mode 2
+  DevBuf<GroupDev> grp;
+  DevBuf<GsnDev> gsn;
+  DevBuf<uint32_t> g_rows, g_fwd_ptr, g_fwd, g_kids, gl_vbase, gl_snbase, gl_inst, g_queue;
+  DevBuf<uint2> g_subs, g_items_fwd, g_items_bwd, g_pack;
+  DevBuf<float> g_vals;
+  uint64_t g_bytes = 0;
+  // per topology with groups: what decides which supernodes k_gsweep takes
+  struct GTopoHost {
+    std::vector<uint8_t> taken, insub;     // laid out for the groups; bottom-subtree supernode
+    std::vector<uint32_t> depth, parent, cost;  // cost = s (s + m)
+    std::vector<uint64_t> sub_cost;             // factor entries of each bottom subtree
+    uint32_t sn_off = 0, sub_base = 0, nsub = 0;
+  };
+  std::vector<GTopoHost> gtopo_host;
+  std::vector<uint32_t> group_topo;                 // per group
+  std::vector<std::vector<uint32_t>> group_snbase;  // per group, per lane: the garment's first supernode
+  uint32_t group_limit = kWarpItemLimit;            // largest s (s + m) of a supernode above the subtrees in k_gsweep
   DevBuf<InstRed> red;
   DevBuf<StepParams> prm;
   SelfContactDev self;       // self-contact buffers (allocated on first use)
@@ -214,85 +242,179 @@ namespace {
 
 vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_t n, vistio_batch* b);
 
-// Tasks (tile x chunk) that one phase can spread over the chip's resident warps
-// (148 SMs x 4 blocks x 8 warps). A phase of fewer is as long as its longest
-// item, so its items are cut to one task per warp; the block items of a larger
-// phase grow with it, since every one gathers its own v (up to kItemTasks; 512
-// sheets with 8 / 32 / 64: 14.21 / 12.40 / 12.36 ms per step). From kManyTasks on
-// a warp takes all tiles of its supernode (24 sheets, below the line: 1546 us so,
-// 1493 with a tile per warp) and supernodes of two chunks too (24 sheets 1590 us so,
-// 1546 with a block each; 512 sheets, above it, 12.4 ms so, 13.3 with a block each).
-constexpr uint64_t kPhaseTasks = 148 * 4 * 8;
-constexpr uint64_t kManyTasks = 4 * kPhaseTasks;
-constexpr uint64_t kItemTasks = 64;
-
-// The sweeps' schedule for a warp-item limit, uploaded: every supernode's step
-// as work items (solve_kernels.cuh), in phases of independent supernodes.
-inline uint32_t sweep_form(const vistio_batch* b) { return b->sweep_occ == 5 ? 0u : b->sweep_occ == 4 ? 1u : 2u; }
-cudaError_t schedule(vistio_batch* b, uint32_t limit, cudaStream_t st) {
-  b->warp_limit = limit;
-  const uint32_t n = uint32_t(b->sn_host.size());
-  const uint32_t NW = kFormWarps[sweep_form(b)];
-  auto tiles_of = [](uint32_t rows) { return (rows + kTile - 1) / kTile; };
+// The level schedule of a batch for a warp-item limit: per level, the
+// supernodes for a whole block (heaviest first), then those for one warp
+// (heaviest first). Which of the two sums a supernode is fixed (warp_item at
+// its default), since their backward sums run in different orders and the
+// results must not depend on the schedule; the limit decides which of the
+// warps' supernodes share a unit: one above it has a block's unit for itself.
+// Fills lvl_off / lvl_nb / lvl_nw and returns the items.
+std::vector<uint32_t> schedule_levels(vistio_batch* b, uint32_t limit) {
+  // in sweep mode 2 the garment groups' tree bottoms belong to k_gsweep
+  const bool grouped = b->sweep_mode == 2;
+  auto skip = [&](uint32_t g) { return grouped && b->sn_grouped[g]; };
+  const uint32_t nsub = grouped ? b->n_sub_plain : b->n_sub;
+  uint32_t L = 0;
+  for (auto& t : b->top) L = std::max(L, t.first + 1);
+  std::vector<std::vector<uint32_t>> blk(L), wrp(L);
+  for (auto& t : b->top) {
+    if (skip(t.second)) continue;
+    const SnDev& S = b->sn_host[t.second];
+    (warp_item(S.ncols, S.nrows) ? wrp : blk)[t.first].push_back(t.second);
+  }
   auto weight = [&](uint32_t q) { return uint64_t(b->sn_host[q].ncols) * (b->sn_host[q].ncols + b->sn_host[q].nrows); };
-  auto side_by_side = [&](uint32_t q) {
-    return b->sweep_mode == 2 && b->sn_in_group[q] && (b->sn_height[q] == 0 || weight(q) <= b->group_limit);
+  // heaviest first; equal supernodes of garments of one topology side by side
+  auto heavier = [&](uint32_t a, uint32_t c) {
+    const uint64_t wa = weight(a), wc = weight(c);
+    if (wa != wc) return wa > wc;
+    if (!b->sn_key.empty() && b->sn_key[a] != b->sn_key[c]) return b->sn_key[a] < b->sn_key[c];
+    return a < c;
   };
-  auto before = [&](uint32_t x, uint32_t y) {
-    const uint64_t wx = weight(x), wy = weight(y);
-    const bool gx = side_by_side(x), gy = side_by_side(y);
-    if (gx != gy) return gy;
-    if (wx != wy && !(gx && b->sn_key[x] >> 32 == b->sn_key[y] >> 32)) return wx > wy;
-    if (b->sn_key[x] != b->sn_key[y]) return b->sn_key[x] < b->sn_key[y];
-    return x < y;
-  };
-  uint32_t P = 0;
-  const std::vector<uint32_t>& rank = b->sweep_mode == 1 ? b->sn_depth : b->sn_height;
-  for (uint32_t k = 0; k < n; ++k) P = std::max(P, rank[k] + 1);
-  std::vector<std::vector<uint32_t>> at(P);  // forward order
-  for (uint32_t k = 0; k < n; ++k) at[b->sweep_mode == 1 ? P - 1 - rank[k] : rank[k]].push_back(k);
-  for (auto& list : at) std::stable_sort(list.begin(), list.end(), before);
-  std::vector<SweepItem> items;
-  b->phases.clear();
-  auto emit = [&](int dir, const std::vector<uint32_t>& list) {
-    vistio_batch::Phase L{dir, uint32_t(items.size()), 0, 0};
-    auto tiles_in = [&](const SnDev& S) { return tiles_of(dir == 0 ? S.ncols + S.nrows : S.ncols); };
-    auto chunks_in = [&](const SnDev& S) { return tiles_of(dir == 0 ? S.ncols : S.nrows); };
-    uint64_t tasks = 0;
-    for (uint32_t k : list) tasks += uint64_t(tiles_in(b->sn_host[k])) * chunks_in(b->sn_host[k]);
-    const uint64_t per_item = std::min(kItemTasks, std::max<uint64_t>(NW, tasks * NW / (2 * kPhaseTasks)));
-    for (int pass = 0; pass < 2; ++pass)  // block items first
-      for (uint32_t k : list) {
-        const SnDev& S = b->sn_host[k];
-        const bool warp = warp_item(S.ncols, S.nrows, limit) && (S.ncols <= kTile || tasks > kManyTasks);
-        if (warp != (pass == 1)) continue;
-        if (dir == 1 && S.nrows == 0) continue;  // a root's forward step is its solution
-        const uint32_t tiles = tiles_in(S);
-        const uint32_t per = warp ? (dir == 1 || tasks <= kManyTasks ? 1u : tiles)
-                                  : std::max(1u, uint32_t(per_item / chunks_in(S)));
-        for (uint32_t t = 0; t < tiles; t += per) {
-          items.push_back(SweepItem{dir == 0 ? S.f_off : S.b_off, S.vbase + S.first, S.vbase, S.ncols, S.nrows, S.rows_off,
-                                    S.inst, t, std::min(per, tiles - t), b->sn_pull[k], b->sn_height[k] > 0});
-          ++(warp ? L.nwarp : L.nblock);
-        }
+  std::vector<uint32_t> items;
+  b->lvl_off.clear(); b->lvl_nb.clear(); b->lvl_nw.clear();
+  for (uint32_t l = 0; l < L; ++l) {
+    std::stable_sort(blk[l].begin(), blk[l].end(), heavier);
+    std::stable_sort(wrp[l].begin(), wrp[l].end(), heavier);
+    b->lvl_off.push_back(uint32_t(items.size()));
+    b->lvl_nb.push_back(uint32_t(blk[l].size()));
+    b->lvl_nw.push_back(uint32_t(wrp[l].size()));
+    items.insert(items.end(), blk[l].begin(), blk[l].end());
+    items.insert(items.end(), wrp[l].begin(), wrp[l].end());
+  }
+  b->warp_limit = limit;
+  // k_sweep units in forward order: bottom subtrees by eight, then each level's
+  // block supernodes one by one and its warp supernodes by eight
+  b->units_host.clear();
+  const uint32_t UI = b->unit_items;
+  for (uint32_t q = 0; q < nsub; q += UI)
+    b->units_host.push_back(make_uint2(0u | (std::min(UI, nsub - q) << 2), q));
+  for (uint32_t l = 0; l < L; ++l) {
+    const uint32_t off = b->lvl_off[l], nb = b->lvl_nb[l], nw = b->lvl_nw[l];
+    for (uint32_t i = 0; i < nb; ++i) b->units_host.push_back(make_uint2(1u | (1u << 2), items[off + i]));
+    for (uint32_t i = 0; i < nw;) {
+      const uint32_t cnt = weight(items[off + nb + i]) > limit ? 1u : std::min(UI, nw - i);
+      b->units_host.push_back(make_uint2(2u | (cnt << 2), off + nb + i));
+      i += cnt;
+    }
+  }
+  b->n_units = uint32_t(b->units_host.size());
+  // The forward sweep's critical path runs from the deepest supernodes of the
+  // tallest trees to their roots. Its units: the bottom subtrees as above,
+  // then the top supernodes by depth below their root, deepest first (blocks,
+  // then warp supernodes by eight of one depth), so the tall trees' chains
+  // start while the short trees' supernodes fill the GPU. Children are deeper
+  // than their parent: the order stays topological.
+  {
+    uint32_t D = 0;
+    for (auto& t : b->top) D = std::max(D, b->sn_depth[t.second] + 1);
+    std::vector<std::vector<uint32_t>> dblk(D), dwrp(D);
+    for (auto& t : b->top) {
+      if (skip(t.second)) continue;
+      const SnDev& S = b->sn_host[t.second];
+      (warp_item(S.ncols, S.nrows) ? dwrp : dblk)[b->sn_depth[t.second]].push_back(t.second);
+    }
+    b->units_fwd_host.clear();
+    b->items_fwd_host.clear();
+    for (uint32_t q = 0; q < nsub; q += UI)
+      b->units_fwd_host.push_back(make_uint2(0u | (std::min(UI, nsub - q) << 2), q));
+    for (uint32_t d = D; d-- > 0;) {
+      std::stable_sort(dblk[d].begin(), dblk[d].end(), heavier);
+      std::stable_sort(dwrp[d].begin(), dwrp[d].end(), heavier);
+      for (uint32_t k : dblk[d]) b->units_fwd_host.push_back(make_uint2(1u | (1u << 2), k));
+      for (size_t i = 0; i < dwrp[d].size();) {
+        const uint32_t off = uint32_t(b->items_fwd_host.size());
+        const uint32_t cnt = weight(dwrp[d][i]) > limit ? 1u : uint32_t(std::min<size_t>(UI, dwrp[d].size() - i));
+        b->items_fwd_host.insert(b->items_fwd_host.end(), dwrp[d].begin() + i, dwrp[d].begin() + i + cnt);
+        b->units_fwd_host.push_back(make_uint2(2u | (cnt << 2), off));
+        i += cnt;
       }
-    if (L.nblock + L.nwarp) b->phases.push_back(L);
-  };
-  for (uint32_t p = 0; p < P; ++p) emit(0, at[p]);
-  for (uint32_t p = P; p-- > 0;) emit(1, at[p]);
-  return b->items.upload(items, st);
+    }
+    b->n_units_fwd = uint32_t(b->units_fwd_host.size());
+  }
+  return items;
 }
 
+// Uploads a schedule from schedule_levels (the unit buffer holds the largest
+// possible count, every top supernode its own unit).
+cudaError_t upload_schedule(vistio_batch* b, const std::vector<uint32_t>& items, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (!items.empty()) e = cudaMemcpyAsync(b->lvl_items.p, items.data(), items.size() * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !b->units_host.empty())
+    e = cudaMemcpyAsync(b->df_units.p, b->units_host.data(), b->units_host.size() * sizeof(uint2),
+                        cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !b->units_fwd_host.empty())
+    e = cudaMemcpyAsync(b->df_units_fwd.p, b->units_fwd_host.data(), b->units_fwd_host.size() * sizeof(uint2),
+                        cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !b->items_fwd_host.empty())
+    e = cudaMemcpyAsync(b->df_items_fwd.p, b->items_fwd_host.data(), b->items_fwd_host.size() * 4,
+                        cudaMemcpyHostToDevice, st);
+  return e;
+}
+// The supernodes k_gsweep takes at a limit: every bottom-subtree supernode,
+// and every laid-out supernode above them whose s (s + m) is at most `limit`
+// and all of whose children are taken (closed downwards). Sets the
+// per-supernode flags that keep them out of k_sweep's schedule and uploads
+// k_gsweep's work items: forward, the subtrees, then the supernodes above them
+// deepest first; backward, those shallowest first, then the subtrees. Within
+// a depth the same supernode of every group is adjacent (shared row indices).
+cudaError_t schedule_groups(vistio_batch* b, uint32_t limit, cudaStream_t st) {
+  std::fill(b->sn_grouped.begin(), b->sn_grouped.end(), uint8_t(0));
+  std::vector<std::vector<uint8_t>> act(b->gtopo_host.size());
+  for (size_t t = 0; t < b->gtopo_host.size(); ++t) {
+    const auto& T = b->gtopo_host[t];
+    const uint32_t ns = uint32_t(T.taken.size());
+    std::vector<uint8_t> kids_ok(ns, 1);
+    act[t].assign(ns, 0);
+    for (uint32_t q = 0; q < ns; ++q) {  // children precede their parents
+      act[t][q] = T.insub[q] || (T.taken[q] && kids_ok[q] && T.cost[q] <= limit);
+      if (!act[t][q] && T.parent[q] != UINT32_MAX) kids_ok[T.parent[q]] = 0;
+    }
+  }
+  struct TopItem { uint32_t depth, q, g; };
+  std::vector<TopItem> tops;
+  std::vector<uint2> fwd, bwd;
+  for (uint32_t g = 0; g < b->group_topo.size(); ++g) {
+    const uint32_t t = b->group_topo[g];
+    const auto& T = b->gtopo_host[t];
+    for (uint32_t base : b->group_snbase[g])
+      for (uint32_t q = 0; q < act[t].size(); ++q)
+        if (act[t][q]) b->sn_grouped[base + q] = 1;
+    for (uint32_t q = 0; q < act[t].size(); ++q)
+      if (act[t][q] && !T.insub[q]) tops.push_back(TopItem{T.depth[q], q, g});
+    for (uint32_t i = 0; i < T.nsub; ++i) fwd.push_back(make_uint2(g, (T.sub_base + i) << 1));
+  }
+  // the bottom subtrees longest first: each warp runs about two items, so the
+  // last ones decide when the launch ends
+  std::stable_sort(fwd.begin(), fwd.end(), [&](const uint2& a, const uint2& c) {
+    const auto& Ta = b->gtopo_host[b->group_topo[a.x]];
+    const auto& Tc = b->gtopo_host[b->group_topo[c.x]];
+    return Ta.sub_cost[(a.y >> 1) - Ta.sub_base] > Tc.sub_cost[(c.y >> 1) - Tc.sub_base];
+  });
+  std::stable_sort(tops.begin(), tops.end(), [](const TopItem& a, const TopItem& c) {
+    return a.depth != c.depth ? a.depth > c.depth : a.q != c.q ? a.q < c.q : a.g < c.g;
+  });
+  const size_t nsub_items = fwd.size();
+  for (const TopItem& x : tops) fwd.push_back(make_uint2(x.g, ((b->gtopo_host[b->group_topo[x.g]].sn_off + x.q) << 1) | 1u));
+  for (size_t i = tops.size(); i-- > 0;)
+    bwd.push_back(make_uint2(tops[i].g, ((b->gtopo_host[b->group_topo[tops[i].g]].sn_off + tops[i].q) << 1) | 1u));
+  bwd.insert(bwd.end(), fwd.begin(), fwd.begin() + nsub_items);
+  b->n_gitems_fwd = uint32_t(fwd.size());
+  b->n_gitems_bwd = uint32_t(bwd.size());
+  b->group_limit = limit;
+  cudaError_t e = cudaSuccess;
+  if (!fwd.empty()) e = cudaMemcpyAsync(b->g_items_fwd.p, fwd.data(), fwd.size() * sizeof(uint2), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !bwd.empty())
+    e = cudaMemcpyAsync(b->g_items_bwd.p, bwd.data(), bwd.size() * sizeof(uint2), cudaMemcpyHostToDevice, st);
+  return e;
+}
+
+inline uint64_t pad4(uint64_t n) { return (n + 3) & ~3ull; }
 float estimate_kappa(const vistio_solver_config& c, const InstanceSetup& I);
 
 // Fronts of the device factorization are allocated for groups of garments
 // of at most this many bytes (at least one garment per group); one buffer
 // serves the groups one after another.
 constexpr uint64_t kFrontBudget = 1ull << 30;
-// FP64 entries of one front and its elimination workspace (FrontDev::work_off).
-inline uint64_t front_doubles(uint64_t s, uint64_t m) {
-  return (s + m) * (s + m) + 2 * (s + m) * kPivots + kPivots * kPivots;
-}
 
 // Device bytes one garment occupies in a batch (the sizes pack_batch
 // allocates), plus the self-contact buffers when those are used.
@@ -301,18 +423,17 @@ uint64_t instance_device_bytes(const InstanceSetup& I, bool refine, bool self_co
   uint64_t vals = 0;
   for (const Supernode& X : F.sn) vals += sn_floats(X.ncols, X.nrows);
   const uint64_t V = I.nv, T = I.nt, H = I.nh, R = F.rows.size();
-  uint64_t b = vals * 4 + F.sn.size() * sizeof(SnDev) + R * 4 + (V + 2 * R) * 4 + R * 16;
-  for (const Supernode& X : F.sn)  // work items: at most one per tile
-    b += sizeof(SweepItem) * (uint64_t(X.ncols + X.nrows + kTile - 1) / kTile + (X.ncols + kTile - 1) / kTile);
+  uint64_t b = vals * 4 + F.sn.size() * sizeof(SnDev) + R * 4 + F.fwd_sn.size() * 4 + (V + 1) * 4 +
+               F.sn.size() * 4 + R * 16;
   b += V * (16 * 10 + 4 + 3 + 4 * 3) + T * (16 + 16 + 4 + 36 + 12) + H * (16 + 16 + 8 + 16 + 16) + (V + 1) * 8;
   if (refine || !F.numeric) b += (V + 1) * 4 + I.A_col.size() * 12;
   if (refine) b += V * 32;
-  // building the panels, freed once done (at most kFrontBudget bytes for a batch
-  // of garments that each need less): the fronts and, factored on the host, its
-  // FP64 factor
-  uint64_t fronts = 0;
-  for (const Supernode& X : F.sn) fronts += 8 * front_doubles(X.ncols, X.nrows);
-  b += std::min(fronts, kFrontBudget) + R * 4 + F.sn.size() * 32 + F.vals.size() * 8;
+  if (!F.numeric) {  // the fronts of the device factorization, freed once it is done (at most kFrontBudget
+                     // bytes for a batch of garments that each need less)
+    uint64_t fronts = 0;
+    for (const Supernode& X : F.sn) fronts += 8 * uint64_t(X.ncols + X.nrows) * (X.ncols + X.nrows);
+    b += std::min(fronts, kFrontBudget) + R * 4 + F.sn.size() * 24;
+  }
   if (self_contact) b += V * 32 + T * (4 + 2 * 2 * 16 + 4) + 48 * T * 8 + V * 4 + 16 * V * 4;
   return b + 12 * V;  // whole-batch position staging
 }
@@ -326,165 +447,111 @@ std::vector<int4> make_chunks(const std::vector<uint64_t>& base, const std::vect
   return ch;
 }
 
-// The sweeps' panels of every garment, built on the device: by the numeric
-// FP64 factorization of the garments whose host set-up is symbolic only, from
-// the host's FP64 factor for the others. The batch's supernodes, rows and
-// permuted A are on the device already.
-vistio_status build_panels(vistio_ctx* ctx, vistio_batch* b, vistio_solver* const* solvers, uint32_t n,
-                           const std::vector<InstDev>& hi, const std::vector<SnDev>& sn,
-                           const std::vector<uint32_t>& relmap) {
+// Numeric FP64 factorization, on the device, of the garments whose host
+// set-up is symbolic only (k_front, one block per supernode, one launch per
+// height of the supernodal trees). The batch's supernodes, rows, permuted A
+// and (zeroed) factor values are on the device already.
+vistio_status factor_on_device(vistio_ctx* ctx, vistio_batch* b, vistio_solver* const* solvers, uint32_t n,
+                               const std::vector<InstDev>& hi, const std::vector<SnDev>& sn,
+                               const std::vector<uint32_t>& rows) {
   cudaStream_t st = ctx->stream;
   const uint64_t NSN = sn.size();
-  const std::vector<uint32_t>&parent = b->sn_parent, &height = b->sn_height;
-  std::vector<uint32_t> kid_ptr(NSN + 1, 0), kids;
-  std::vector<uint64_t> front_off(NSN, 0), work_off(NSN, 0), host_p(NSN, 0), host_d(NSN, 0);
-  for (uint64_t g = 0; g < NSN; ++g)
-    if (parent[g] != kNoParent) kid_ptr[parent[g] + 1]++;
+  std::vector<uint32_t> parent(NSN, UINT32_MAX), height(NSN, 0), kid_ptr(NSN + 1, 0), kids, relmap(rows.size(), 0);
+  std::vector<uint64_t> front_off(NSN, 0);
+  for (uint32_t k = 0; k < n; ++k) {
+    const Factor& F = solvers[k]->setup.factor;
+    if (F.numeric) continue;
+    const uint32_t base = hi[k].sn_base;
+    for (uint32_t q = 0; q < F.sn.size(); ++q) {
+      if (F.sn[q].parent == UINT32_MAX) continue;
+      const uint32_t g = base + q, p = base + F.sn[q].parent;
+      parent[g] = p;
+      kid_ptr[p + 1]++;
+      height[p] = std::max(height[p], height[g] + 1);  // children precede parents
+    }
+  }
   for (uint64_t g = 0; g < NSN; ++g) kid_ptr[g + 1] += kid_ptr[g];
   kids.resize(kid_ptr[NSN]);
   {
     std::vector<uint32_t> cur(kid_ptr.begin(), kid_ptr.end() - 1);
     for (uint64_t g = 0; g < NSN; ++g)
-      if (parent[g] != kNoParent) kids[cur[parent[g]]++] = uint32_t(g);
+      if (parent[g] != UINT32_MAX) kids[cur[parent[g]]++] = uint32_t(g);
   }
-  // Groups of garments of one kind; per group the launches in order: fronts from
-  // the host's factor at once, or by height assemble, then the elimination
-  // steps; then the panels.
-  enum Kind : uint32_t { kAssemble, kPivot, kUpdate, kFromHost, kEmit };
-  struct Launch { Kind kind; uint32_t step, first, count; };
-  std::vector<uint2> items;
-  std::vector<Launch> launches;
-  std::vector<double> host_vals;
-  uint64_t gsize = 0, max_gsize = 0, max_host = 0;
+  // each child row's position in its parent's front: a column of the parent
+  // or one of the parent's rows (the child's rows are a subset of those)
+  for (uint64_t g = 0; g < NSN; ++g) {
+    if (parent[g] == UINT32_MAX) continue;
+    const SnDev &C = sn[g], &P = sn[parent[g]];
+    const uint32_t* Rp = rows.data() + P.rows_off;
+    for (uint32_t j = 0; j < C.nrows; ++j) {
+      const uint32_t r = rows[C.rows_off + j];
+      uint32_t at;
+      if (r >= P.first && r < P.first + P.ncols) {
+        at = r - P.first;
+      } else {
+        const uint32_t* it = std::lower_bound(Rp, Rp + P.nrows, r);
+        if (it == Rp + P.nrows || *it != r)
+          return fail(ctx, VISTIO_ERR_INVARIANT, "supernode rows are not contained in the parent's front");
+        at = P.ncols + uint32_t(it - Rp);
+      }
+      relmap[C.rows_off + j] = at;
+    }
+  }
+  // groups of garments, and per group the supernodes by height
+  std::vector<uint32_t> items;
+  std::vector<uint2> launches;  // (first item, count)
+  uint64_t gsize = 0, max_gsize = 0;
   std::vector<uint32_t> group;
-  bool group_numeric = false;
-  struct HostPart { size_t launch, first, count; };
-  std::vector<HostPart> uploads;  // host factors to copy before a launch
-  auto add = [&](Kind kind, uint32_t step, size_t first) {
-    if (items.size() > first) launches.push_back({kind, step, uint32_t(first), uint32_t(items.size() - first)});
-  };
-  auto tiles = [](uint64_t x, uint32_t t) { return uint32_t((x + t - 1) / t); };
   auto flush = [&]() {
     if (group.empty()) return;
-    auto each = [&](auto fn) {
+    uint32_t hmax = 0;
+    for (uint32_t k : group)
+      for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) hmax = std::max(hmax, height[g]);
+    for (uint32_t h = 0; h <= hmax; ++h) {
+      const uint32_t first = uint32_t(items.size());
       for (uint32_t k : group)
-        for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) fn(g, sn[g].ncols, sn[g].ncols + sn[g].nrows);
-    };
-    size_t first;
-    if (group_numeric) {
-      uploads.push_back({launches.size(), 0, 0});
-      uploads.back().first = host_vals.size();
-      for (uint32_t k : group) {
-        const Factor& F = solvers[k]->setup.factor;
-        const uint64_t base = host_vals.size() - uploads.back().first;
-        for (uint32_t q = 0; q < hi[k].nsn; ++q) {
-          host_p[hi[k].sn_base + q] = base + F.sn[q].panel_off;
-          host_d[hi[k].sn_base + q] = base + F.sn[q].diag_off;
-        }
-        host_vals.insert(host_vals.end(), F.vals.begin(), F.vals.end());
-      }
-      uploads.back().count = host_vals.size() - uploads.back().first;
-      max_host = std::max<uint64_t>(max_host, uploads.back().count);
-      first = items.size();
-      each([&](uint32_t g, uint32_t s, uint32_t nf) {
-        for (uint32_t i = 0; i < tiles(nf, 32); ++i)
-          for (uint32_t j = 0; j < tiles(s, 32) && j <= i; ++j) items.push_back(make_uint2(g, i << 16 | j));
-      });
-      add(kFromHost, 0, first);
-    } else {
-      uint32_t hmax = 0;
-      each([&](uint32_t g, uint32_t, uint32_t) { hmax = std::max(hmax, height[g]); });
-      std::vector<std::vector<uint32_t>> at(hmax + 1);
-      each([&](uint32_t g, uint32_t, uint32_t) { at[height[g]].push_back(g); });
-      for (uint32_t h = 0; h <= hmax; ++h) {
-        first = items.size();
-        uint32_t smax = 0;
-        for (uint32_t g : at[h]) {
-          smax = std::max(smax, sn[g].ncols);
-          for (uint32_t i = 0; i < tiles(sn[g].ncols + sn[g].nrows, kAssembleRows); ++i) items.push_back(make_uint2(g, i));
-        }
-        add(kAssemble, 0, first);
-        for (uint32_t t = 0; t * kPivots < smax; ++t) {
-          first = items.size();
-          for (uint32_t g : at[h])
-            if (sn[g].ncols > t * kPivots)
-              for (uint32_t i = 0; i < tiles(sn[g].ncols + sn[g].nrows, kPivotRows); ++i) items.push_back(make_uint2(g, i));
-          add(kPivot, t, first);
-          first = items.size();
-          for (uint32_t g : at[h])
-            if (sn[g].ncols > t * kPivots)
-              for (uint32_t i = 0; i < tiles(sn[g].ncols + sn[g].nrows, kUpdateTile); ++i)
-                for (uint32_t j = 0; j <= i; ++j) items.push_back(make_uint2(g, i << 16 | j));
-          add(kUpdate, t, first);
-        }
-      }
+        for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g)
+          if (height[g] == h) items.push_back(g);
+      if (items.size() > first) launches.push_back(make_uint2(first, uint32_t(items.size()) - first));
     }
-    first = items.size();
-    each([&](uint32_t g, uint32_t, uint32_t nf) {
-      for (uint32_t i = 0; i < tiles(nf, 32); ++i) items.push_back(make_uint2(g, i));
-    });
-    add(kEmit, 0, first);
     max_gsize = std::max(max_gsize, gsize);
     group.clear();
     gsize = 0;
   };
-  for (int numeric = 0; numeric < 2; ++numeric) {
-    for (uint32_t k = 0; k < n; ++k) {
-      if (solvers[k]->setup.factor.numeric != (numeric != 0)) continue;
-      uint64_t fb = 0;
-      for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) {
-        if (uint64_t(sn[g].ncols) + sn[g].nrows >= 65536)
-          return fail(ctx, VISTIO_ERR_CAPACITY, "supernode front too large for the device factorization");
-        fb += front_doubles(sn[g].ncols, sn[g].nrows);
-      }
-      if (!group.empty() && (gsize + fb) * 8 > kFrontBudget) flush();
-      for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) {
-        const uint64_t nf = uint64_t(sn[g].ncols) + sn[g].nrows;
-        front_off[g] = gsize;
-        work_off[g] = gsize + nf * nf;
-        gsize += front_doubles(sn[g].ncols, sn[g].nrows);
-      }
-      group.push_back(k);
-      group_numeric = numeric != 0;
+  for (uint32_t k = 0; k < n; ++k) {
+    if (solvers[k]->setup.factor.numeric) continue;
+    uint64_t fb = 0;
+    for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) {
+      const uint64_t nf = uint64_t(sn[g].ncols) + sn[g].nrows;
+      if (nf >= 65536) return fail(ctx, VISTIO_ERR_CAPACITY, "supernode front too large for the device factorization");
+      fb += nf * nf;
     }
-    flush();
+    if (!group.empty() && (gsize + fb) * 8 > kFrontBudget) flush();
+    for (uint32_t g = hi[k].sn_base; g < hi[k].sn_base + hi[k].nsn; ++g) {
+      const uint64_t nf = uint64_t(sn[g].ncols) + sn[g].nrows;
+      front_off[g] = gsize;
+      gsize += nf * nf;
+    }
+    group.push_back(k);
   }
-  DevBuf<uint32_t> d_kid_ptr, d_kids, d_relmap, d_status;
-  DevBuf<uint64_t> d_front_off, d_work_off, d_host_p, d_host_d;
-  DevBuf<uint2> d_items;
-  DevBuf<double> d_fronts, d_host;
+  flush();
+  DevBuf<uint32_t> d_kid_ptr, d_kids, d_relmap, d_items, d_status;
+  DevBuf<uint64_t> d_front_off;
+  DevBuf<double> d_fronts;
   CU(d_kid_ptr.upload(kid_ptr, st)); CU(d_kids.upload(kids, st)); CU(d_relmap.upload(relmap, st));
-  CU(d_items.upload(items, st)); CU(d_front_off.upload(front_off, st)); CU(d_work_off.upload(work_off, st));
-  if (max_host) { CU(d_host_p.upload(host_p, st)); CU(d_host_d.upload(host_d, st)); CU(d_host.alloc(max_host, st)); }
+  CU(d_items.upload(items, st)); CU(d_front_off.upload(front_off, st));
   CU(d_fronts.alloc(max_gsize, st));
   CU(d_status.alloc(1, st)); CU(cudaMemsetAsync(d_status.p, 0, sizeof(uint32_t), st));
   FrontDev D;
   D.sn = b->sn.p; D.rows = b->rows.p;
   D.a_ptr = b->a_ptr.p; D.a_col = b->a_col.p; D.a_val = b->a_val.p;
-  D.front_off = d_front_off.p; D.work_off = d_work_off.p; D.kid_ptr = d_kid_ptr.p; D.kids = d_kids.p;
-  D.relmap = d_relmap.p; D.host_p = d_host_p.p; D.host_d = d_host_d.p; D.host_vals = d_host.p;
-  D.fronts = d_fronts.p; D.work = d_fronts.p; D.vals = b->vals.p; D.status = d_status.p;
+  D.front_off = d_front_off.p; D.kid_ptr = d_kid_ptr.p; D.kids = d_kids.p; D.relmap = d_relmap.p;
+  D.fronts = d_fronts.p; D.vals = b->vals.p; D.status = d_status.p;
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   CU(cudaEventRecord(e0, st));
-  size_t up = 0;
-  bool on_device = false;
-  for (size_t l = 0; l < launches.size(); ++l) {
-    if (up < uploads.size() && uploads[up].launch == l) {
-      CU(cudaMemcpyAsync(d_host.p, host_vals.data() + uploads[up].first, uploads[up].count * 8, cudaMemcpyHostToDevice, st));
-      ++up;
-    }
-    const Launch& L = launches[l];
-    const uint2* it = d_items.p + L.first;
-    switch (L.kind) {
-      case kAssemble: k_fassemble<<<L.count, 256, 0, st>>>(D, it); on_device = true; break;
-      case kPivot: k_fpivot<<<L.count, kPivotRows, 0, st>>>(D, it, L.step); break;
-      case kUpdate: k_fupdate<<<L.count, 256, 0, st>>>(D, it, L.step); break;
-      case kFromHost: k_ffrom_host<<<L.count, 256, 0, st>>>(D, it); break;
-      case kEmit: k_femit<<<L.count, 256, 0, st>>>(D, it); break;
-    }
-  }
+  for (const uint2& L : launches) k_front<<<L.y, kFrontThreads, 0, st>>>(D, d_items.p + L.x);
   CU(cudaGetLastError());
   CU(cudaEventRecord(e1, st));
   uint32_t status = 0;
@@ -494,20 +561,19 @@ vistio_status build_panels(vistio_ctx* ctx, vistio_batch* b, vistio_solver* cons
   CU(cudaEventElapsedTime(&ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  b->factor_ms = ms;
   if (status & 32u) return fail(ctx, VISTIO_ERR_NOT_SPD, "matrix is not symmetric positive definite (device Cholesky pivot)");
-  if (on_device) {  // 0, 0 if every garment was factored on the host
-    b->factor_ms = ms;
-    b->factor_launches = uint32_t(launches.size());
-  }
+  if (status & 64u) return fail(ctx, VISTIO_ERR_INVARIANT, "matrix entry outside the symbolic factor structure");
+  b->factor_launches = uint32_t(launches.size());
   return VISTIO_OK;
 }
 
 // True if two factors have one symbolic structure: the same ordering
-// outcome, supernodes, row structures, elimination tree and pull lists (only
-// the numbers may differ).
+// outcome, supernodes, row structures, elimination tree, bottom subtrees and
+// pull lists (only the numbers may differ).
 bool same_structure(const Factor& a, const Factor& b) {
   if (a.n != b.n || a.sn.size() != b.sn.size() || a.rows.size() != b.rows.size() || a.nlevels != b.nlevels ||
-      a.fwd_sn.size() != b.fwd_sn.size())
+      a.sub_first.size() != b.sub_first.size() || a.fwd_sn.size() != b.fwd_sn.size())
     return false;
   auto eq = [](const std::vector<uint32_t>& x, const std::vector<uint32_t>& y) {
     return x.size() == y.size() && (x.empty() || std::memcmp(x.data(), y.data(), x.size() * 4) == 0);
@@ -518,38 +584,84 @@ bool same_structure(const Factor& a, const Factor& b) {
         x.parent != y.parent || x.level != y.level)
       return false;
   }
-  return eq(a.rows, b.rows) && eq(a.fwd_ptr, b.fwd_ptr) && eq(a.fwd_sn, b.fwd_sn) && eq(a.fwd_pos, b.fwd_pos);
+  return eq(a.rows, b.rows) && eq(a.sub_first, b.sub_first) && eq(a.sub_last, b.sub_last) && eq(a.fwd_ptr, b.fwd_ptr) &&
+         eq(a.fwd_sn, b.fwd_sn) && eq(a.fwd_pos, b.fwd_pos);
 }
 
 // The garment groups of a batch: garments of one symbolic structure (a
-// topology), in batch order, kGroupLanes per group; a remainder of fewer than
-// kGroupMinLanes garments stays ungrouped.
-constexpr uint32_t kGroupLanes = 32, kGroupMinLanes = 8;
+// topology), in batch order, kGroupLanes per group; a remainder of fewer
+// than kGroupMinLanes garments stays ungrouped. Per topology, the supernodes
+// k_gsweep takes: every bottom-subtree supernode, and every supernode of at
+// most kWarpVec columns within the default warp-item limit all of whose
+// children are taken (so the taken set is closed downwards).
 struct GroupPlan {
-  std::vector<uint8_t> grouped;  // per garment
+  struct Topo {
+    uint32_t leader = 0;
+    std::vector<uint32_t> members;
+    std::vector<uint8_t> taken, insub;
+    std::vector<uint32_t> depth;  // supernodes above each one
+    uint64_t entries = 0;         // interleaved entries of one group's value block
+    uint32_t sn_off = 0, row_base = 0, sub_base = 0, rows_base = 0, fwd_base = 0;
+  };
+  std::vector<Topo> topos;
+  std::vector<int32_t> group;  // per garment: its group, or -1
+  std::vector<uint32_t> lane;  // per garment: its lane in the group
   std::vector<uint32_t> sclass;  // per garment: its symbolic structure class (any size)
-  uint32_t groups = 0;
+  std::vector<uint32_t> gtopo; // per group: its topology
+  std::vector<std::vector<uint32_t>> gmembers;
 };
 
 GroupPlan plan_groups(vistio_solver* const* solvers, uint32_t n) {
   GroupPlan G;
-  G.grouped.assign(n, 0);
+  G.group.assign(n, -1);
+  G.lane.assign(n, 0);
   G.sclass.assign(n, 0);
-  std::vector<std::vector<uint32_t>> members;  // per class
+  std::vector<GroupPlan::Topo> all;
   for (uint32_t k = 0; k < n; ++k) {
     const Factor& F = solvers[k]->setup.factor;
     size_t t = 0;
-    for (; t < members.size(); ++t)
-      if (same_structure(solvers[members[t][0]]->setup.factor, F)) break;
-    if (t == members.size()) members.emplace_back();
-    members[t].push_back(k);
+    for (; t < all.size(); ++t)
+      if (same_structure(solvers[all[t].leader]->setup.factor, F)) break;
+    if (t == all.size()) {
+      all.emplace_back();
+      all.back().leader = k;
+    }
+    all[t].members.push_back(k);
     G.sclass[k] = uint32_t(t);
   }
-  for (const auto& m : members)
-    for (size_t i = 0; i < m.size() && m.size() - i >= kGroupMinLanes; i += kGroupLanes) {
-      ++G.groups;
-      for (size_t l = i; l < std::min<size_t>(m.size(), i + kGroupLanes); ++l) G.grouped[m[l]] = 1;
+  for (auto& T : all) {
+    if (T.members.size() < kGroupMinLanes) continue;
+    const Factor& F = solvers[T.leader]->setup.factor;
+    const uint32_t ns = uint32_t(F.sn.size());
+    T.insub.assign(ns, 0);
+    for (size_t q = 0; q < F.sub_first.size(); ++q)
+      for (uint32_t k = F.sub_first[q]; k <= F.sub_last[q]; ++k) T.insub[k] = 1;
+    T.taken.assign(ns, 0);
+    std::vector<uint8_t> kids_taken(ns, 1);
+    for (uint32_t q = 0; q < ns; ++q) {  // children precede their parents
+      const Supernode& X = F.sn[q];
+      T.taken[q] = T.insub[q] ||
+                   (kids_taken[q] && X.ncols <= kWarpVec && uint64_t(X.ncols) * (X.ncols + X.nrows) <= kWarpItemLimit);
+      if (X.parent != UINT32_MAX && !T.taken[q]) kids_taken[X.parent] = 0;
+      if (T.taken[q]) T.entries += uint64_t(X.ncols) * (X.ncols + 1) / 2 + uint64_t(X.nrows) * X.ncols;
     }
+    T.depth.assign(ns, 0);
+    for (uint32_t q = ns; q-- > 0;)
+      if (F.sn[q].parent != UINT32_MAX) T.depth[q] = T.depth[F.sn[q].parent] + 1;
+    const uint32_t ti = uint32_t(G.topos.size());
+    for (size_t i = 0; i < T.members.size(); i += kGroupLanes) {
+      const uint32_t cnt = uint32_t(std::min<size_t>(kGroupLanes, T.members.size() - i));
+      if (cnt < kGroupMinLanes) break;
+      const uint32_t g = uint32_t(G.gmembers.size());
+      G.gmembers.emplace_back(T.members.begin() + i, T.members.begin() + i + cnt);
+      G.gtopo.push_back(ti);
+      for (uint32_t l = 0; l < cnt; ++l) {
+        G.group[T.members[i + l]] = int32_t(g);
+        G.lane[T.members[i + l]] = l;
+      }
+    }
+    G.topos.push_back(std::move(T));
+  }
   return G;
 }
 
@@ -562,10 +674,11 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   // untuned: sixteen-warp sweep blocks for a few garments (their solves are
   // one tree's chains), four eight-warp blocks per SM otherwise
   b->sweep_occ = n <= kWideMaxInstances ? 2u : 4u;
+  b->unit_items = b->sweep_occ == 2 ? 2 * kUnitItems : kUnitItems;
   b->cfg = solvers[0]->cfg;
   std::vector<InstDev> hi(n);
   std::vector<uint64_t> vb(n), vc(n), tb(n), tc(n), hb(n), hc(n);
-  uint64_t V = 0, T = 0, H = 0, NSN = 0, NROWS = 0, NVALS = 0;
+  uint64_t V = 0, T = 0, H = 0, NSN = 0, NROWS = 0, NVALS = 0, NLVL = 0, NFWD = 0;
   for (uint32_t k = 0; k < n; ++k) {
     const InstanceSetup& I = solvers[k]->setup;
     vb[k] = V; vc[k] = I.nv; tb[k] = T; tc[k] = I.nt; hb[k] = H; hc[k] = I.nh;
@@ -582,6 +695,7 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
       if (I.hinge_st[q] != ((q & 3u) < 2u ? -1.f : 1.f)) d.unit_stencils = 0;
     V += I.nv; T += I.nt; H += I.nh; NSN += I.factor.sn.size(); NROWS += I.factor.rows.size();
     for (const Supernode& X : I.factor.sn) NVALS += sn_floats(X.ncols, X.nrows);
+    NLVL += I.factor.nlevels + 1; NFWD += I.factor.fwd_sn.size();
   }
   if (V >= (1ull << 31) || 3 * T >= (1ull << 30) || 4 * H >= (1ull << 30))
     return fail(ctx, VISTIO_ERR_CAPACITY, "batch too large for 32-bit element indices");
@@ -596,23 +710,38 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   std::vector<uint4> hinge_idx(H);
   std::vector<float4> hinge_st(H);
   std::vector<float2> hinge_wr(H);
-  std::vector<uint32_t> vtri_ptr, vhinge_ptr, perm_local(V), rows;
+  std::vector<uint32_t> vtri_ptr, vhinge_ptr, perm_local(V), fwd_ptr(V + 1, 0), rows;
   std::vector<uint32_t> vtri, vhinge;  // incidence, per connectivity class
   std::vector<SnDev> sn(NSN);
+  std::vector<float> vals(NVALS + 4, 0.f);  // +16 bytes: staging windows round up to 16 bytes
+  std::vector<uint32_t> fwd(NFWD);
   rows.reserve(NROWS);
-  const GroupPlan gp = plan_groups(solvers, n);
-  if (NROWS >= (1ull << 32)) return fail(ctx, VISTIO_ERR_CAPACITY, "batch too large for 32-bit U slot indices");
-  b->sn_key.assign(NSN, 0);
-  b->sn_parent.assign(NSN, kNoParent);
-  b->sn_height.assign(NSN, 0);
-  b->sn_depth.assign(NSN, 0);
-  b->sn_in_group.assign(NSN, 0);
-  uint64_t snb = 0, rowsb = 0, valsb = 0;
+  uint32_t LMAX = 0;
+  for (uint32_t k = 0; k < n; ++k) LMAX = std::max(LMAX, solvers[k]->setup.factor.nlevels);
+  (void)LMAX;
+  std::vector<uint2> subs, subs_grouped;
+  // Garment groups, and the U slots of every garment: ungrouped garments
+  // first, one contiguous run each; then per group 32 slots per local slot,
+  // lane-minor (slot i of lane l at u_base + i * 32 + l)
+  GroupPlan gp = plan_groups(solvers, n);
+  std::vector<uint64_t> ubase(n, 0), g_ubase(gp.gmembers.size(), 0);
+  uint64_t NU = 0;
+  for (uint32_t k = 0; k < n; ++k)
+    if (gp.group[k] < 0) { ubase[k] = NU; NU += solvers[k]->setup.factor.rows.size(); }
+  for (size_t g = 0; g < gp.gmembers.size(); ++g) {
+    g_ubase[g] = NU;
+    NU += uint64_t(kGroupLanes) * solvers[gp.gmembers[g][0]]->setup.factor.rows.size();
+  }
+  if (NU >= (1ull << 32)) return fail(ctx, VISTIO_ERR_CAPACITY, "batch too large for 32-bit U slot indices");
+  uint64_t snb = 0, rowsb = 0, valsb = 0, fwdb = 0;
   for (uint32_t k = 0; k < n; ++k) {
     vistio_solver* S = solvers[k];
     const InstanceSetup& I = S->setup;
     const Factor& F = I.factor;
     uint64_t v0 = vb[k], t0 = tb[k], h0 = hb[k];
+    const bool grouped = gp.group[k] >= 0;
+    const uint64_t ub = grouped ? g_ubase[gp.group[k]] + gp.lane[k] : ubase[k];
+    const uint32_t us = grouped ? kGroupLanes : 1u;  // U slot of local slot i: ub + i * us
     for (uint32_t i = 0; i < I.nv; ++i) {
       pos[v0 + i] = make_float4(S->host_pos[3 * i], S->host_pos[3 * i + 1], S->host_pos[3 * i + 2], 0.f);
       vel[v0 + i] = make_float4(S->host_vel[3 * i], S->host_vel[3 * i + 1], S->host_vel[3 * i + 2], 0.f);
@@ -632,70 +761,41 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
       hinge_st[h0 + h] = make_float4(I.hinge_st[4 * h], I.hinge_st[4 * h + 1], I.hinge_st[4 * h + 2], I.hinge_st[4 * h + 3]);
       hinge_wr[h0 + h] = make_float2(I.hinge_w[h], I.hinge_rest[h]);
     }
-    // per supernode its two panels (see SnDev), written by build_panels, and its
-    // place in the tree
+    // factor: per supernode one 16-byte aligned region [D | P] (see SnDev)
     for (size_t q = 0; q < F.sn.size(); ++q) {
       const Supernode& X = F.sn[q];
-      const uint64_t g = snb + q;
-      SnDev& d = sn[g];
-      d.first = X.first; d.ncols = X.ncols; d.nrows = X.nrows;
+      SnDev& d = sn[snb + q];
+      const uint32_t sc = X.ncols, m = X.nrows;
+      d.first = X.first; d.ncols = sc; d.nrows = m;
       d.rows_off = uint32_t(rowsb + X.rows_off);
-      d.f_off = valsb;
-      d.b_off = valsb + X.ncols * pad8(X.nrows + X.ncols);
-      valsb += sn_floats(X.ncols, X.nrows);
+      const uint32_t ld = sn_ld(sc);  // odd leading dimension of D and P (bank-conflict-free reads)
+      d.d_off = valsb; valsb += pad4(uint64_t(sc) * ld);
+      d.p_off = valsb; valsb += pad4(uint64_t(m) * ld + m);  // panel, then its row indices
       d.vbase = uint32_t(v0);
       d.inst = k;
-      b->sn_key[g] = (uint64_t(gp.sclass[k]) << 32) | q;
-      b->sn_in_group[g] = gp.grouped[k];
-      if (X.parent == UINT32_MAX) continue;
-      b->sn_parent[g] = uint32_t(snb) + X.parent;  // children precede parents
-      b->sn_height[snb + X.parent] = std::max(b->sn_height[snb + X.parent], b->sn_height[g] + 1);
-    }
-    for (size_t q = F.sn.size(); q-- > 0;)
-      if (F.sn[q].parent != UINT32_MAX) b->sn_depth[snb + q] = b->sn_depth[snb + F.sn[q].parent] + 1;
-    rows.insert(rows.end(), F.rows.begin(), F.rows.end());
-    snb += F.sn.size(); rowsb += F.rows.size();
-  }
-  // Each child row's position in its parent's front (a column of the parent or
-  // one of its rows: the child's rows are a subset of those), and the inverse:
-  // per front position the children's slots there, in child order.
-  std::vector<uint32_t> relmap(NROWS), pull_ptr, pull(NROWS);
-  b->sn_pull.assign(NSN, 0);
-  {
-    uint64_t lists = 0;
-    for (uint64_t g = 0; g < NSN; ++g) {
-      b->sn_pull[g] = uint32_t(lists);
-      lists += sn[g].ncols + sn[g].nrows;
-    }
-    if (lists >= (1ull << 32)) return fail(ctx, VISTIO_ERR_CAPACITY, "batch too large for 32-bit pull lists");
-    pull_ptr.assign(lists + 1, 0);
-    for (uint64_t g = 0; g < NSN; ++g) {
-      const uint32_t p = b->sn_parent[g];
-      if (p == kNoParent) continue;
-      const SnDev &C = sn[g], &P = sn[p];
-      const uint32_t* Rp = rows.data() + P.rows_off;
-      for (uint32_t j = 0, at = 0; j < C.nrows; ++j) {  // both lists ascend
-        const uint32_t r = rows[C.rows_off + j];
-        uint32_t& pos = relmap[C.rows_off + j];
-        if (r >= P.first && r < P.first + P.ncols) {
-          pos = r - P.first;
-        } else {
-          while (at < P.nrows && Rp[at] < r) ++at;
-          if (at == P.nrows || Rp[at] != r)
-            return fail(ctx, VISTIO_ERR_INVARIANT, "supernode rows are not contained in the parent's front");
-          pos = P.ncols + at;
-        }
-        pull_ptr[b->sn_pull[p] + pos + 1]++;
+      d.u_off = uint32_t(ub + uint64_t(X.rows_off) * us);
+      d.u_stride = us;
+      if (X.level != kBottomLevel) b->top.push_back({X.level, uint32_t(snb + q)});
+      if (F.numeric) {  // else the device factorization writes D and P
+        const double* Pn = F.vals.data() + X.panel_off;   // row-major m x s
+        const double* Dn = F.vals.data() + X.diag_off;    // column-major s x s
+        for (uint64_t j = 0; j < m; ++j)
+          for (uint32_t c = 0; c < sc; ++c) vals[d.p_off + j * ld + c] = float(Pn[j * sc + c]);
+        for (uint64_t c = 0; c < sc; ++c)
+          for (uint32_t i = 0; i < sc; ++i) vals[d.d_off + c * ld + i] = float(Dn[c * sc + i]);
       }
+      // the panel's row indices (u32 bits), staged with the panel by the sweeps
+      std::memcpy(vals.data() + d.p_off + uint64_t(m) * ld, F.rows.data() + X.rows_off, size_t(m) * 4);
     }
-    for (uint64_t i = 0; i < lists; ++i) pull_ptr[i + 1] += pull_ptr[i];
-    std::vector<uint32_t> fill(pull_ptr.begin(), pull_ptr.end() - 1);
-    for (uint64_t g = 0; g < NSN; ++g)
-      if (b->sn_parent[g] != kNoParent)
-        for (uint32_t j = 0; j < sn[g].nrows; ++j)
-          pull[fill[b->sn_pull[b->sn_parent[g]] + relmap[sn[g].rows_off + j]]++] = sn[g].rows_off + j;
-    pull.resize(pull_ptr.back());
+    rows.insert(rows.end(), F.rows.begin(), F.rows.end());
+    for (size_t q = 0; q < F.sub_first.size(); ++q)
+      (grouped ? subs_grouped : subs).push_back(make_uint2(uint32_t(snb + F.sub_first[q]), uint32_t(snb + F.sub_last[q])));
+    for (uint32_t r = 0; r < I.nv; ++r) fwd_ptr[v0 + r] = uint32_t(fwdb + F.fwd_ptr[r]);
+    for (size_t q = 0; q < F.fwd_sn.size(); ++q)
+      fwd[fwdb + q] = uint32_t(ub + uint64_t(F.sn[F.fwd_sn[q]].rows_off + F.fwd_pos[q]) * us);
+    snb += F.sn.size(); rowsb += F.rows.size(); fwdb += F.fwd_sn.size();
   }
+  fwd_ptr[V] = uint32_t(fwdb);
   // f64 CSR of each instance's A with rows and columns in solve order (global ids)
   std::vector<uint32_t> a_ptr, a_col;
   std::vector<double> a_val;
@@ -716,6 +816,42 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
     b->refine = b->cfg.refinement_sweeps;
   }
   b->sn_host = sn;
+  b->sn_key.assign(NSN, 0);
+  for (uint32_t k = 0; k < n; ++k)
+    for (uint32_t q = 0; q < hi[k].nsn; ++q) b->sn_key[hi[k].sn_base + q] = (uint64_t(gp.sclass[k]) << 32) | q;
+  // subtree units take eight consecutive subtrees: the same subtree of
+  // garments of one topology side by side (equal work for the block's warps)
+  auto by_key = [&](const uint2& a, const uint2& c) {
+    return b->sn_key[a.x] != b->sn_key[c.x] ? b->sn_key[a.x] < b->sn_key[c.x] : a.x < c.x;
+  };
+  std::sort(subs.begin(), subs.end(), by_key);
+  std::sort(subs_grouped.begin(), subs_grouped.end(), by_key);
+  b->n_sub_plain = uint32_t(subs.size());
+  subs.insert(subs.end(), subs_grouped.begin(), subs_grouped.end());
+  b->n_sub = uint32_t(subs.size());
+  // the supernodal tree for the dependency-driven sweeps (global ids)
+  std::vector<uint32_t> df_parent(NSN, kNoParent), df_nkids(NSN, 0), df_kid_ptr(NSN + 1, 0), df_kids;
+  for (uint32_t k = 0; k < n; ++k) {
+    const Factor& F = solvers[k]->setup.factor;
+    const uint32_t base = hi[k].sn_base;
+    for (uint32_t q = 0; q < F.sn.size(); ++q)
+      if (F.sn[q].parent != UINT32_MAX) {
+        df_parent[base + q] = base + F.sn[q].parent;
+        df_nkids[base + F.sn[q].parent]++;
+      }
+  }
+  // depth below the root: parents come after their children (postorder)
+  b->sn_depth.assign(NSN, 0);
+  for (uint64_t g = NSN; g-- > 0;)
+    if (df_parent[g] != kNoParent) b->sn_depth[g] = b->sn_depth[df_parent[g]] + 1;
+  std::vector<uint32_t> items = schedule_levels(b, b->warp_limit);
+  for (uint64_t g = 0; g < NSN; ++g) df_kid_ptr[g + 1] = df_kid_ptr[g] + df_nkids[g];
+  df_kids.resize(df_kid_ptr[NSN]);
+  {
+    std::vector<uint32_t> cur(df_kid_ptr.begin(), df_kid_ptr.end() - 1);
+    for (uint64_t g = 0; g < NSN; ++g)
+      if (df_parent[g] != kNoParent) df_kids[cur[df_parent[g]]++] = uint32_t(g);
+  }
   // Vertex incidence, once per connectivity class: garments with the same
   // triangles and hinges (the batched workload's garments of one grid side)
   // share one list of (local element << 2 | slot) codes and one array of
@@ -774,13 +910,24 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   CU(b->vhinge_ptr.upload(vhinge_ptr, st)); CU(b->vhinge.upload(vhinge, st));
   CU(b->perm_local.upload(perm_local, st));
   CU(b->Y.alloc(V, st)); CU(b->Tm.alloc(V, st));
-  CU(b->sn.upload(sn, st)); CU(b->rows.upload(rows, st)); CU(b->vals.alloc(NVALS, st));
-  CU(b->pull_ptr.upload(pull_ptr, st)); CU(b->pull.upload(pull, st));
-  CU(b->U.alloc(NROWS, st));
+  CU(b->sn.upload(sn, st)); CU(b->rows.upload(rows, st)); CU(b->vals.upload(vals, st));
+  CU(b->lvl_items.upload(items, st));
+  CU(b->sub_items.upload(subs, st));
+  CU(b->df_units.alloc((b->n_sub + kSolveWarps - 1) / kSolveWarps + b->top.size() + 1, st));
+  CU(b->df_units_fwd.alloc((b->n_sub + kSolveWarps - 1) / kSolveWarps + b->top.size() + 1, st));
+  CU(b->df_items_fwd.alloc(b->top.size() + 1, st));
+  CU(upload_schedule(b, items, st));
+  CU(b->df_parent.upload(df_parent, st)); CU(b->df_nkids.upload(df_nkids, st));
+  CU(b->df_kid_ptr.upload(df_kid_ptr, st)); CU(b->df_kids.upload(df_kids, st));
+  CU(b->df_cnt.alloc(NSN, st)); CU(cudaMemsetAsync(b->df_cnt.p, 0, NSN * 4, st));
+  CU(b->df_flag.alloc(NSN, st)); CU(cudaMemsetAsync(b->df_flag.p, 0, NSN * 4, st));
+  CU(b->df_queue.alloc(2, st)); CU(cudaMemsetAsync(b->df_queue.p, 0, 8, st));
+  CU(b->fwd_ptr.upload(fwd_ptr, st)); CU(b->fwd.upload(fwd, st));
+  CU(b->U.alloc(NU, st));
   if (have_a) { CU(b->a_ptr.upload(a_ptr, st)); CU(b->a_col.upload(a_col, st)); CU(b->a_val.upload(a_val, st)); }
   if (b->refine) { CU(b->R0.alloc(V, st)); CU(b->W.alloc(V, st)); }
-  {
-    vistio_status r = build_panels(ctx, b, solvers, n, hi, sn, relmap);
+  if (on_device) {
+    vistio_status r = factor_on_device(ctx, b, solvers, n, hi, sn, rows);
     if (r != VISTIO_OK) return r;
     if (!b->refine) { b->a_ptr.reset(); b->a_col.reset(); b->a_val.reset(); }
   }
@@ -793,8 +940,11 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   CU(b->prm.alloc(1, st));
   CU(b->status.alloc(1, st)); CU(cudaMemsetAsync(b->status.p, 0, sizeof(uint32_t), st));
   CU(cudaStreamSynchronize(st));
-  b->factor_bytes = NVALS * sizeof(float) + sn.size() * sizeof(SnDev) + rows.size() * 4 + pull.size() * 4 +
-                    pull_ptr.size() * 4 + rows.size() * 16;
+  b->factor_bytes = vals.size() * sizeof(float) + sn.size() * sizeof(SnDev) + rows.size() * 4 + fwd.size() * 4 +
+                    fwd_ptr.size() * 4 + items.size() * 4 + rows.size() * 16;
+  b->device_bytes = b->factor_bytes + V * (16 * 10 + 4 + 3 + 4 * 3) + T * (16 + 16 + 4 + 36 + 12) +
+                    H * (16 + 16 + 8 + 16 + 16) + (V + 1) * 8 + NSN * 28 + b->df_units.n * 8;
+  if (b->refine) b->device_bytes += (V + 1) * 4 + a_col.size() * 12 + V * 32;
   BatchDev& d = b->dev;
   d.inst = b->inst.p; d.tri_chunks = b->tri_chunks.p; d.hinge_chunks = b->hinge_chunks.p; d.vtx_chunks = b->vtx_chunks.p;
   d.pos = b->pos.p; d.vel = b->vel.p; d.prev = b->prev.p; d.pred = b->pred.p; d.mass = b->mass.p; d.pinned = b->pinned.p;
@@ -802,21 +952,127 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   d.hinge_idx = b->hinge_idx.p; d.hinge_st = b->hinge_st.p; d.hinge_wr = b->hinge_wr.p; d.hinge_out = b->hinge_out.p;
   d.vtri_ptr = b->vtri_ptr.p; d.vtri = b->vtri.p; d.vhinge_ptr = b->vhinge_ptr.p; d.vhinge = b->vhinge.p;
   d.perm_local = b->perm_local.p; d.row_vertex = nullptr; d.Y = b->Y.p; d.T = b->Tm.p;
-  d.sn = b->sn.p; d.rows = b->rows.p; d.vals = b->vals.p;
-  d.pull_ptr = b->pull_ptr.p; d.pull = b->pull.p; d.U = b->U.p;
+  d.sn = b->sn.p; d.rows = b->rows.p; d.vals = b->vals.p; d.lvl_items = b->lvl_items.p; d.sub_items = b->sub_items.p;
+  d.fwd_ptr = b->fwd_ptr.p; d.fwd = b->fwd.p; d.U = b->U.p;
+  d.df_units = b->df_units.p; d.df_parent = b->df_parent.p; d.df_nkids = b->df_nkids.p;
+  d.df_units_fwd = b->df_units_fwd.p; d.df_items_fwd = b->df_items_fwd.p;
+  d.df_kid_ptr = b->df_kid_ptr.p; d.df_kids = b->df_kids.p; d.df_cnt = b->df_cnt.p; d.df_flag = b->df_flag.p;
+  d.df_queue = b->df_queue.p;
   d.a_ptr = b->a_ptr.p; d.a_col = b->a_col.p; d.a_val = b->a_val.p; d.R0 = b->R0.p; d.W = b->W.p;
   d.grad = b->grad.p; d.grad_up = b->grad_up.p; d.lam = b->lam.p; d.fin_n = b->fin_n.p;
   d.in_contact = b->in_contact.p; d.in_contact_up = b->in_contact_up.p; d.ever = b->ever.p;
   d.red = b->red.p; d.prm = b->prm.p; d.status = b->status.p;
-  b->n_groups = gp.groups;
-  if (b->n_groups) b->sweep_mode = 2;
+  // ---- garment groups: topology tables, lanes, interleaved values, work items
+  b->n_groups = uint32_t(gp.gmembers.size());
+  b->sn_grouped.assign(NSN, 0);
+  if (b->n_groups) {
+    std::vector<GsnDev> gsn;
+    std::vector<uint32_t> g_rows, g_fwd_ptr, g_fwd, g_kids;
+    std::vector<uint2> g_subs;
+    for (auto& T : gp.topos) {
+      const Factor& F = solvers[T.leader]->setup.factor;
+      const uint32_t ns = uint32_t(F.sn.size());
+      T.sn_off = uint32_t(gsn.size());
+      T.rows_base = uint32_t(g_rows.size());
+      T.row_base = uint32_t(g_fwd_ptr.size());
+      T.fwd_base = uint32_t(g_fwd.size());
+      T.sub_base = uint32_t(g_subs.size());
+      std::vector<std::vector<uint32_t>> kids(ns);
+      for (uint32_t q = 0; q < ns; ++q)
+        if (F.sn[q].parent != UINT32_MAX) kids[F.sn[q].parent].push_back(q);
+      uint64_t goff = 0;
+      for (uint32_t q = 0; q < ns; ++q) {
+        const Supernode& X = F.sn[q];
+        GsnDev g{};
+        g.first = X.first; g.ncols = X.ncols; g.nrows = X.nrows;
+        g.rows_off = T.rows_base + X.rows_off;
+        g.u_local = X.rows_off;
+        g.parent = X.parent == UINT32_MAX ? kGNone : X.parent;
+        g.kid_off = uint32_t(g_kids.size());
+        g.nkids = uint32_t(kids[q].size());
+        g_kids.insert(g_kids.end(), kids[q].begin(), kids[q].end());
+        g.g_off = goff;
+        if (T.taken[q]) goff += uint64_t(X.ncols) * (X.ncols + 1) / 2 + uint64_t(X.nrows) * X.ncols;
+        gsn.push_back(g);
+      }
+      g_rows.insert(g_rows.end(), F.rows.begin(), F.rows.end());
+      for (uint32_t r = 0; r <= F.n; ++r) g_fwd_ptr.push_back(T.fwd_base + F.fwd_ptr[r]);
+      for (size_t q = 0; q < F.fwd_sn.size(); ++q) g_fwd.push_back(F.sn[F.fwd_sn[q]].rows_off + F.fwd_pos[q]);
+      for (size_t q = 0; q < F.sub_first.size(); ++q)
+        g_subs.push_back(make_uint2(T.sn_off + F.sub_first[q], T.sn_off + F.sub_last[q]));
+    }
+    const uint32_t NG = b->n_groups;
+    std::vector<GroupDev> grp(NG);
+    std::vector<uint32_t> gl_vbase(kGroupLanes * NG, 0), gl_snbase(kGroupLanes * NG, 0), gl_inst(kGroupLanes * NG, 0);
+    std::vector<uint2> pack;
+    uint64_t gbase = 0, max_items = 0;
+    for (const auto& T : gp.topos) {
+      vistio_batch::GTopoHost h;
+      const Factor& F = solvers[T.leader]->setup.factor;
+      h.taken = T.taken; h.insub = T.insub; h.depth = T.depth;
+      h.sn_off = T.sn_off; h.sub_base = T.sub_base; h.nsub = uint32_t(F.sub_first.size());
+      for (const Supernode& X : F.sn) {
+        h.parent.push_back(X.parent);
+        h.cost.push_back(X.ncols * (X.ncols + X.nrows));
+      }
+      for (size_t q = 0; q < F.sub_first.size(); ++q) {
+        uint64_t c = 0;
+        for (uint32_t k = F.sub_first[q]; k <= F.sub_last[q]; ++k)
+          c += uint64_t(F.sn[k].ncols) * (F.sn[k].ncols + 1) / 2 + uint64_t(F.sn[k].nrows) * F.sn[k].ncols;
+        h.sub_cost.push_back(c);
+      }
+      b->gtopo_host.push_back(std::move(h));
+    }
+    for (uint32_t g = 0; g < NG; ++g) {
+      const auto& T = gp.topos[gp.gtopo[g]];
+      const auto& mem = gp.gmembers[g];
+      grp[g] = GroupDev{T.sn_off, uint32_t(mem.size()), gbase, uint32_t(g_ubase[g]), T.row_base};
+      gbase += T.entries;
+      b->group_topo.push_back(gp.gtopo[g]);
+      b->group_snbase.emplace_back();
+      for (uint32_t l = 0; l < mem.size(); ++l) {
+        const uint32_t k = mem[l];
+        gl_vbase[kGroupLanes * g + l] = uint32_t(vb[k]);
+        gl_snbase[kGroupLanes * g + l] = hi[k].sn_base;
+        gl_inst[kGroupLanes * g + l] = k;
+        b->group_snbase.back().push_back(hi[k].sn_base);
+      }
+      for (uint32_t q = 0; q < T.taken.size(); ++q) {
+        if (!T.taken[q]) continue;
+        pack.push_back(make_uint2(g, T.sn_off + q));
+        ++max_items;  // a supernode above the subtrees, or part of one subtree item
+      }
+    }
+    b->n_gpack = uint32_t(pack.size());
+    CU(b->grp.upload(grp, st)); CU(b->gsn.upload(gsn, st));
+    CU(b->g_rows.upload(g_rows, st)); CU(b->g_fwd_ptr.upload(g_fwd_ptr, st)); CU(b->g_kids.upload(g_kids, st));
+    CU(b->g_fwd.upload(g_fwd, st));
+    CU(b->g_subs.upload(g_subs, st));
+    CU(b->gl_vbase.upload(gl_vbase, st)); CU(b->gl_snbase.upload(gl_snbase, st)); CU(b->gl_inst.upload(gl_inst, st));
+    CU(b->g_items_fwd.alloc(max_items + 1, st)); CU(b->g_items_bwd.alloc(max_items + 1, st));
+    CU(b->g_pack.upload(pack, st));
+    CU(b->g_queue.alloc(2, st)); CU(cudaMemsetAsync(b->g_queue.p, 0, 8, st));
+    CU(b->g_vals.alloc(gbase * kGroupLanes, st));
+    d.grp = b->grp.p; d.gsn = b->gsn.p; d.g_rows = b->g_rows.p; d.g_fwd_ptr = b->g_fwd_ptr.p; d.g_fwd = b->g_fwd.p;
+    d.g_kids = b->g_kids.p; d.g_subs = b->g_subs.p; d.gl_vbase = b->gl_vbase.p; d.gl_snbase = b->gl_snbase.p;
+    d.gl_inst = b->gl_inst.p; d.g_vals = b->g_vals.p; d.g_items_fwd = b->g_items_fwd.p;
+    d.g_items_bwd = b->g_items_bwd.p; d.g_queue = b->g_queue.p;
+    // the groups' factor values, interleaved from the per-garment regions
+    if (!pack.empty()) k_gpack<<<uint32_t(pack.size()), 256, 0, st>>>(d, b->g_vals.p, b->g_pack.p);
+    CU(cudaGetLastError());
+    CU(cudaStreamSynchronize(st));
+    b->g_bytes = gbase * kGroupLanes * 4 + gsn.size() * sizeof(GsnDev) + (g_rows.size() + g_fwd_ptr.size() +
+                 g_fwd.size() + g_kids.size()) * 4 + (2 * max_items + pack.size()) * 8;
+    b->device_bytes += b->g_bytes;
+    b->g_pack.reset();
+    b->sweep_mode = 2;
+    CU(schedule_groups(b, b->group_limit, st));
+    std::vector<uint32_t> items2 = schedule_levels(b, b->warp_limit);
+    CU(upload_schedule(b, items2, st));
+    CU(cudaStreamSynchronize(st));
+  }
   b->dev_w = d;
   b->dev_w.Y = b->W.p;
-  CU(schedule(b, b->warp_limit, st));
-  CU(cudaStreamSynchronize(st));
-  b->device_bytes = b->factor_bytes + V * (16 * 10 + 4 + 3 + 4 * 3) + T * (16 + 16 + 4 + 36 + 12) +
-                    H * (16 + 16 + 8 + 16 + 16) + (V + 1) * 8 + b->items.n * sizeof(SweepItem);
-  if (b->refine) b->device_bytes += (V + 1) * 4 + a_col.size() * 12 + V * 32;
   return VISTIO_OK;
 }
 
@@ -877,20 +1133,53 @@ StepParams make_params(const vistio_solver_config& c, float dt, const vistio_con
   return p;
 }
 
-// Both sweeps over the whole batch: right-hand side dv.T, solution dv.Y, one
-// launch per phase. Returns the launches.
-uint32_t launch_sweeps(vistio_batch* b, const BatchDev& dv, cudaStream_t st) {
-  using Kernel = void (*)(BatchDev, const SweepItem*, uint32_t, uint32_t);
-  static const Kernel kernels[kForms][2] = {
-      {k_level<0, 0>, k_level<1, 0>}, {k_level<0, 1>, k_level<1, 1>}, {k_level<0, 2>, k_level<1, 2>}};
-  const uint32_t form = sweep_form(b), NW = kFormWarps[form];
-  for (const auto& L : b->phases)
-    launch_pdl(kernels[form][L.dir], L.nblock + (L.nwarp + NW - 1) / NW, 32 * NW, level_smem(NW), st, dv,
-               static_cast<const SweepItem*>(b->items.p + L.off), L.nblock, L.nwarp);
-  return uint32_t(b->phases.size());
+// One k_sweep launch over the batch's units in the chosen compiled form.
+void launch_k_sweep(vistio_batch* b, const BatchDev& dv, cudaStream_t st) {
+  const uint32_t form = b->sweep_occ == 5 ? 0u : b->sweep_occ == 4 ? 1u : 2u;
+  const uint32_t grid = std::min(b->n_units_fwd + b->n_units, b->ctx->sweep_blocks[form]);
+  if (form == 0) launch_pdl(k_sweep<5>, grid, kSolveThreads, kSolveSmem, st, dv, b->n_units_fwd, b->n_units);
+  else if (form == 1) launch_pdl(k_sweep<4>, grid, kSolveThreads, kSolveSmem, st, dv, b->n_units_fwd, b->n_units);
+  else
+    launch_pdl(k_sweep<2, kWideWarps>, grid, 32 * kWideWarps, kWideSmem, st, dv, b->n_units_fwd, b->n_units);
 }
 
-// One FP64 refinement: T = R0 - A d, then the sweeps solve A W = T.
+// Forward then backward sweep, level by level over the whole batch, in place
+// on dv.Y (right-hand side in, solution out). Returns the launches.
+uint32_t launch_sweeps(vistio_batch* b, const BatchDev& dv, cudaStream_t st) {
+  if (b->sweep_mode == 2 && b->n_groups) {
+    // the groups' tree bottoms forward, everything above them (and the
+    // ungrouped garments) both ways, then the groups' tree bottoms backward
+    const uint32_t gf = std::min((b->n_gitems_fwd + kGWarps - 1) / kGWarps, b->ctx->gsweep_blocks);
+    const uint32_t gb = std::min((b->n_gitems_bwd + kGWarps - 1) / kGWarps, b->ctx->gsweep_blocks);
+    uint32_t n = 0;
+    if (gf) { launch_pdl(k_gsweep<0>, gf, kGThreads, kGSmem, st, dv, b->n_gitems_fwd); ++n; }
+    if (b->n_units_fwd + b->n_units) {
+      launch_k_sweep(b, dv, st);
+      ++n;
+    }
+    if (gb) { launch_pdl(k_gsweep<1>, gb, kGThreads, kGSmem, st, dv, b->n_gitems_bwd); ++n; }
+    return n;
+  }
+  if (b->sweep_mode == 1 && b->n_units) {
+    launch_k_sweep(b, dv, st);
+    return 1;
+  }
+  uint32_t L = uint32_t(b->lvl_off.size()), n = 0;
+  const uint32_t sub_grid = (b->n_sub + kSolveWarps - 1) / kSolveWarps;
+  if (sub_grid) { launch_pdl(k_subtree<0>, sub_grid, kSolveThreads, kSolveSmem, st, dv, b->n_sub); ++n; }
+  for (uint32_t l = 0; l < L; ++l) {
+    uint32_t grid = b->lvl_nb[l] + (b->lvl_nw[l] + kSolveWarps - 1) / kSolveWarps;
+    if (grid) { launch_pdl(k_level<0>, grid, kSolveThreads, kSolveSmem, st, dv, b->lvl_off[l], b->lvl_nb[l], b->lvl_nw[l]); ++n; }
+  }
+  for (int l = int(L) - 1; l >= 0; --l) {
+    uint32_t grid = b->lvl_nb[l] + (b->lvl_nw[l] + kSolveWarps - 1) / kSolveWarps;
+    if (grid) { launch_pdl(k_level<1>, grid, kSolveThreads, kSolveSmem, st, dv, b->lvl_off[l], b->lvl_nb[l], b->lvl_nw[l]); ++n; }
+  }
+  if (sub_grid) { launch_pdl(k_subtree<1>, sub_grid, kSolveThreads, kSolveSmem, st, dv, b->n_sub); ++n; }
+  return n;
+}
+
+// One FP64 refinement: W = R0 - A d, then the sweeps solve A e = W in place.
 uint32_t launch_refinement(vistio_batch* b, cudaStream_t st) {
   launch_pdl(k_refine, b->n_vtx_chunks, kElemThreads, 0, st, b->dev);
   return 1 + launch_sweeps(b, b->dev_w, st);
@@ -1171,12 +1460,27 @@ vistio_status vistio_ctx_create(int32_t device, vistio_ctx** out) {
     uint64_t keep = UINT64_MAX;
     CU(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
   }
-  CU(cudaFuncSetAttribute(k_level<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[0])));
-  CU(cudaFuncSetAttribute(k_level<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[0])));
-  CU(cudaFuncSetAttribute(k_level<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[1])));
-  CU(cudaFuncSetAttribute(k_level<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[1])));
-  CU(cudaFuncSetAttribute(k_level<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[2])));
-  CU(cudaFuncSetAttribute(k_level<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, level_smem(kFormWarps[2])));
+  CU(cudaFuncSetAttribute(k_level<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_level<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_subtree<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_subtree<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_sweep<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  CU(cudaFuncSetAttribute(k_sweep<2, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
+  CU(cudaFuncSetAttribute(k_gsweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
+  CU(cudaFuncSetAttribute(k_gsweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
+  {
+    int per_sm = 0, sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<5>, kSolveThreads, kSolveSmem));
+    c->sweep_blocks[0] = uint32_t(std::max(1, per_sm) * std::max(1, sms));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<4>, kSolveThreads, kSolveSmem));
+    c->sweep_blocks[1] = uint32_t(std::max(1, per_sm) * std::max(1, sms));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep<2, kWideWarps>, 32 * kWideWarps, kWideSmem));
+    c->sweep_blocks[2] = uint32_t(std::max(1, per_sm) * std::max(1, sms));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gsweep<0>, kGThreads, kGSmem));
+    c->gsweep_blocks = uint32_t(std::max(1, per_sm) * std::max(1, sms));
+  }
   *out = c.release();
   return VISTIO_OK;
 }
@@ -1582,12 +1886,11 @@ vistio_status vistio_batch_launches_per_step(const vistio_batch* b, uint32_t* la
 
 void* vistio_batch_stream(vistio_batch* b) { return b ? (void*)b->ctx->stream : nullptr; }
 
-// Sweep autotuner. The candidates are the orders of the work (by height, by
-// depth, groups side by side) times the warp-item limits of s (s + m): 0 (every
-// supernode for a block) ... 2^30 (every one of at most kWarpCols columns
-// for a warp), and for the grouped order the group limits.
+// Sweep autotuner. The candidates are the two sweep kinds (one launch per
+// level; dependency-driven) times the warp-item limits of s (s + m): 0 (every
+// warp's supernode a unit for itself) ... 2^30 (all of them in shared units).
 static const uint32_t kTuneLimits[7] = {0u, 1024u, 2048u, 4096u, 6144u, 12288u, 1u << 30};
-// Group limits of the grouped kind's candidates: 0 takes the leaves only.
+// Group limits of the grouped kind's candidates: 0 takes the bottom subtrees only.
 static const uint32_t kGroupTuneLimits[7] = {0u, 64u, 128u, 256u, 512u, 1024u, 6144u};
 
 namespace {
@@ -1612,7 +1915,7 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
   uint32_t best_limit = b->warp_limit, best_mode = b->sweep_mode, best_glimit = b->group_limit;
   uint32_t best1_limit = kWarpItemLimit;  // the fastest limit of kind 1: kind 2 runs its rest at it
   b->sweep_occ = 4;
-  CU(cudaMemsetAsync(b->Tm.p, 0, b->V * sizeof(float4), st));
+  b->unit_items = kUnitItems;
   for (int c = 0; c < 21; ++c) {
     const uint32_t glimit = c >= 14 ? kGroupTuneLimits[c - 14] : b->group_limit;
     if (c >= 14 && (!b->n_groups || glimit > best1_limit)) {  // no groups, or a limit kind 1's rest could not match
@@ -1621,8 +1924,10 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
     }
     b->sweep_mode = uint32_t(c / 7);
     const uint32_t limit = c >= 14 ? best1_limit : kTuneLimits[c % 7];
-    b->group_limit = glimit;
-    CU(schedule(b, limit, st));
+    if (c >= 14) CU(schedule_groups(b, glimit, st));
+    std::vector<uint32_t> items = schedule_levels(b, limit);
+    CU(upload_schedule(b, items, st));
+    CU(cudaMemsetAsync(b->Y.p, 0, b->V * sizeof(float4), st));
     launch_sweeps(b, b->dev, st);  // warm-up
     CU(cudaEventRecord(e0, st));
     for (int r = 0; r < 3; ++r) launch_sweeps(b, b->dev, st);
@@ -1638,18 +1943,21 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
   uint32_t status = 0;
   CU(cudaMemcpyAsync(&status, b->status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
   b->sweep_mode = best_mode;
-  b->group_limit = best_glimit;
-  CU(schedule(b, best_limit, st));
-  {
-    // the chosen schedule with k_level's three compiled forms (five and four
-    // eight-warp blocks per SM, two sixteen-warp blocks): the fastest is kept
+  if (b->n_groups) CU(schedule_groups(b, best_glimit, st));
+  std::vector<uint32_t> items = schedule_levels(b, best_limit);
+  CU(upload_schedule(b, items, st));
+  if (best_mode != 0) {
+    // the chosen schedule with k_sweep's three compiled forms (five and four
+    // eight-warp blocks per SM, two sixteen-warp blocks with units of twice
+    // the items): the fastest is kept
     float occ_ms[3] = {0.f, 0.f, 0.f};
-    auto use = [&](int v) {
-      b->sweep_occ = v == 0 ? 5u : v == 1 ? 4u : 2u;
-      return schedule(b, best_limit, st);
-    };
     for (int v = 0; v < 3; ++v) {
-      CU(use(v));
+      b->sweep_occ = v == 0 ? 5u : v == 1 ? 4u : 2u;
+      if (v == 2) {
+        b->unit_items = 2 * kUnitItems;
+        std::vector<uint32_t> wide = schedule_levels(b, best_limit);
+        CU(upload_schedule(b, wide, st));
+      }
       launch_sweeps(b, b->dev, st);  // warm-up
       CU(cudaEventRecord(e0, st));
       for (int r = 0; r < 3; ++r) launch_sweeps(b, b->dev, st);
@@ -1661,9 +1969,16 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
     int bv = 0;
     for (int v = 1; v < 3; ++v)
       if (occ_ms[v] < occ_ms[bv]) bv = v;
-    CU(use(bv));
+    b->sweep_occ = bv == 0 ? 5u : bv == 1 ? 4u : 2u;
+    if (bv != 2) {  // back to eight-warp units
+      b->unit_items = kUnitItems;
+      std::vector<uint32_t> narrow = schedule_levels(b, best_limit);
+      CU(upload_schedule(b, narrow, st));
+    }
     best = occ_ms[bv];
     for (int v = 0; v < 3; ++v) b->occ_ms[v] = occ_ms[v];
+  } else {
+    b->sweep_occ = 4;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1679,8 +1994,9 @@ vistio_status vistio_batch_set_group_limit(vistio_batch* b, uint32_t limit) {
   if (!b) return fail(nullptr, VISTIO_ERR_INVALID_CONFIG, "null batch");
   vistio_ctx* ctx = b->ctx;
   if (!b->n_groups) return fail(ctx, VISTIO_ERR_INVALID_CONFIG, "the batch has no garment groups");
-  b->group_limit = std::min(limit, kWarpItemLimit);
-  CU(schedule(b, b->warp_limit, ctx->stream));
+  CU(schedule_groups(b, std::min(limit, kWarpItemLimit), ctx->stream));
+  std::vector<uint32_t> items = schedule_levels(b, b->warp_limit);
+  CU(upload_schedule(b, items, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   return drop_graphs(b);
 }
@@ -1746,7 +2062,8 @@ vistio_status vistio_batch_set_self_ccd_dedup(vistio_batch* b, uint32_t on) {
 vistio_status vistio_batch_set_warp_limit(vistio_batch* b, uint32_t limit) {
   if (!b) return fail(nullptr, VISTIO_ERR_INVALID_CONFIG, "null batch");
   vistio_ctx* ctx = b->ctx;
-  CU(schedule(b, limit, ctx->stream));
+  std::vector<uint32_t> items = schedule_levels(b, limit);
+  CU(upload_schedule(b, items, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   return drop_graphs(b);
 }
@@ -1758,7 +2075,8 @@ vistio_status vistio_batch_set_sweep_mode(vistio_batch* b, uint32_t mode) {
     return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "sweep mode 2 needs garment groups (none in this batch)");
   vistio_ctx* ctx = b->ctx;
   b->sweep_mode = mode;
-  CU(schedule(b, b->warp_limit, ctx->stream));
+  std::vector<uint32_t> items = schedule_levels(b, b->warp_limit);  // mode 2 leaves the groups' supernodes out
+  CU(upload_schedule(b, items, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   return drop_graphs(b);
 }
@@ -1766,11 +2084,16 @@ vistio_status vistio_batch_set_sweep_mode(vistio_batch* b, uint32_t mode) {
 vistio_status vistio_batch_set_sweep_blocks(vistio_batch* b, uint32_t blocks_per_sm) {
   if (!b) return fail(nullptr, VISTIO_ERR_INVALID_CONFIG, "null batch");
   if (blocks_per_sm != 2 && blocks_per_sm != 4 && blocks_per_sm != 5)
-    return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "k_level is compiled for 5 or 4 eight-warp blocks or 2 sixteen-warp blocks per SM");
+    return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "k_sweep is compiled for 5 or 4 eight-warp blocks or 2 sixteen-warp blocks per SM");
   vistio_ctx* ctx = b->ctx;
   b->sweep_occ = blocks_per_sm;
-  CU(schedule(b, b->warp_limit, ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
+  const uint32_t ui = blocks_per_sm == 2 ? 2 * kUnitItems : kUnitItems;
+  if (ui != b->unit_items) {
+    b->unit_items = ui;
+    std::vector<uint32_t> items = schedule_levels(b, b->warp_limit);
+    CU(upload_schedule(b, items, b->ctx->stream));
+    CU(cudaStreamSynchronize(b->ctx->stream));
+  }
   return drop_graphs(b);
 }
 
@@ -1817,7 +2140,7 @@ vistio_status vistio_batch_phase_bytes(const vistio_batch* b, int32_t phase, uin
   if (!b || !bytes) return fail(nullptr, VISTIO_ERR_INVALID_CONFIG, "null argument");
   uint64_t V = b->V, T = b->T, H = b->H, stored = 0, fwd = 0, rows = 0;
   for (auto* s : b->solvers) {
-    for (const Supernode& X : s->setup.factor.sn) stored += uint64_t(X.ncols) * (X.ncols + 2ull * X.nrows);
+    stored += s->setup.factor.nnz_stored;
     fwd += s->setup.factor.fwd_sn.size();
     rows += s->setup.factor.rows.size();
   }
@@ -1826,13 +2149,13 @@ vistio_status vistio_batch_phase_bytes(const vistio_batch* b, int32_t phase, uin
     case 1: *bytes = T * (16 + 16 + 4 + 36) + 3 * T * 16; break; // indices, Dm^-1, w, 3 contributions; 3 gathered x
     case 2: *bytes = H * (16 + 16 + 8 + 16) + 4 * H * 16; break; // indices, stencil, (w, theta0), out; 4 gathered x
     case 3: *bytes = V * (4 + 16 + 16 + 16) + (V + 1) * 8 + 3 * T * (4 + 12) + 4 * H * (4 + 16 + 4); break;
-    case 4: *bytes = 4 * stored + fwd * 4 + rows * (4 + 2 * 16) + V * (2 * 16 + 2 * 16) + V * 8; break;
+    case 4: *bytes = 2 * 4 * stored + fwd * 4 + rows * (4 + 2 * 16) + V * (2 * 16 + 2 * 16) + V * 8; break;
     case 5: *bytes = V * (16 * 3 + 1 + 16); break;
     case 6: {  // refinement: A (f64 value + column), d gathered, R0, W; then one sweep pair
       uint64_t nnz_a = 0;
       for (auto* s : b->solvers) nnz_a += s->setup.A_col.size();
       *bytes = nnz_a * 12 + (V + 1) * 4 + V * (16 + 16 + 16) +
-               4 * stored + fwd * 4 + rows * (4 + 2 * 16) + V * (2 * 16 + 2 * 16);
+               2 * 4 * stored + fwd * 4 + rows * (4 + 2 * 16) + V * (2 * 16 + 2 * 16);
       break;
     }
     default: return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "unknown phase");
@@ -1883,7 +2206,7 @@ vistio_status vistio_sparse_factorize(vistio_ctx* ctx, uint32_t n, const uint32_
   std::vector<double> sym_val = f->A_val;
   mirror_upper(n, sym_ptr, sym_col, sym_val);
   // the host finds the ordering and the symbolic structure; the numeric
-  // factorization runs on the device when the batch is packed
+  // factorization runs on the device (k_front) when the batch is packed
   int st = 0;
   std::string err = factorize_csr(n, sym_ptr.data(), sym_col.data(), sym_val.data(), nullptr, f->f, &st, false);
   if (!err.empty()) return fail(ctx, st == 11 ? VISTIO_ERR_NOT_SPD : VISTIO_ERR_INVALID_CONFIG, err);
@@ -1926,7 +2249,7 @@ vistio_status vistio_sparse_solve(vistio_factor* f, const float* rhs, float* sol
   std::vector<float4> y(n);
   for (int pass = 0; pass < 3; ++pass) {
     for (uint32_t i = 0; i < n; ++i) y[f->f.iperm[i]] = make_float4(float(r[i]), 0.f, 0.f, 0.f);
-    CU(cudaMemcpyAsync(b->Tm.p, y.data(), n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
+    CU(cudaMemcpyAsync(b->Y.p, y.data(), n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
     launch_solve(b, ctx->stream, After::kSums, 0, true);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(y.data(), b->Y.p, n * sizeof(float4), cudaMemcpyDeviceToHost, ctx->stream));
