@@ -2492,6 +2492,7 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
   launch_self_sort(d, S.view(), uint32_t(ch.size()), st);
   launch_self_boxes(d, S.view(), uint32_t(ch.size()), margin, st);
   launch_self_pairs(d, S.view(), uint32_t(ch.size()), st);
+  CU(cudaGetLastError());  // before the count is read: without the launches it is zero
   uint32_t total = 0;
   CU(cudaMemcpyAsync(&total, S.npairs, 4, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
@@ -2504,6 +2505,7 @@ vistio_status broadphase_pairs_impl(vistio_ctx* ctx, uint32_t nv, const float* p
     CU(cudaMallocAsync(reinterpret_cast<void**>(&S.pairs), uint64_t(total) * sizeof(uint2), st));
     CU(cudaMemsetAsync(S.npairs, 0, 4, st));
     launch_self_pairs(d, S.view(), uint32_t(ch.size()), st);
+    CU(cudaGetLastError());
   }
   DevBuf<uint32_t> row;
   CU(row.alloc(total, st));
