@@ -304,13 +304,17 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
  * counterpart): triangles per thread of the membrane step (1: 256 threads
  * per chunk of 256 triangles; 2: 128 threads, both triangles' loads issued
  * first) and hinges per thread of the bending step (the same two shapes),
- * each timed over five launches; the faster of each pair is kept. The shapes
- * compute the same arithmetic per element: results are bit-identical.
+ * each timed over five launches; the faster of each pair is kept. Batches of at
+ * most 2,368 chunks of 256 elements can also run both steps in one launch, one
+ * element per thread: it is timed too, and kept if it takes less than the two.
+ * The shapes compute the same arithmetic per element: results are bit-identical.
  * candidate_ms (4 entries, may be NULL): membrane 1, 2, bending 1, 2. Without
- * tuning: 2 triangles and 1 hinge per thread. Synchronises the stream. */
+ * tuning: both steps in one launch where that can be, else 2 triangles and 1
+ * hinge per thread. Synchronises the stream. */
 vistio_status vistio_batch_tune_local(vistio_batch* b, uint32_t* tri_per_thread, uint32_t* hinge_per_thread,
                                       float* candidate_ms);
-/* Sets the local steps' elements per thread directly (1 or 2 each). */
+/* Sets the local steps' elements per thread directly (1 or 2 each); each step
+ * is then a launch of its own, whatever the batch's size. */
 vistio_status vistio_batch_set_local_shape(vistio_batch* b, uint32_t tri_per_thread, uint32_t hinge_per_thread);
 /* How the self-contact CCD step bound (compute_max_step_size,
  * crates/vistio-contact/src/ccd.rs:238-292) visits its vertex-triangle tests.
@@ -352,9 +356,10 @@ vistio_status vistio_batch_launches_per_step(const vistio_batch* b, uint32_t* la
 /* The stream the batch runs on (cudaStream_t as void*), for event timing. */
 void* vistio_batch_stream(vistio_batch* b);
 /* Launches one kernel phase of a plain PD iteration on the batch stream, for
- * per-kernel timing: 0 predict, 1 local membrane, 2 local bending, 3 residual
- * gather, 4 forward + back substitution (no position update), 5 finalize.
- * Uses the step constants of the last vistio_batch_step call. Asynchronous. */
+ * per-kernel timing: 0 predict, 1 local membrane, 2 local bending (each as a
+ * launch of its own, also where the step runs both in one), 3 residual gather,
+ * 4 forward + back substitution (no position update), 5 finalize. Uses the step
+ * constants of the last vistio_batch_step call. Asynchronous. */
 vistio_status vistio_batch_launch_phase(vistio_batch* b, int32_t phase);
 /* Algorithmic bytes of one launch of a phase over the whole batch (see
  * vistio_batch_launch_phase), from the batch's element counts and factor sizes:

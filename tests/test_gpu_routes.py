@@ -74,3 +74,21 @@ def test_batched_steps_bitwise_equal_the_garment_alone(count):
             continue  # two garments are no group
         for got in run(count, mode, blocks):
             assert np.array_equal(got, alone), (mode, blocks)
+
+
+def test_local_shapes_that_are_set_are_run():
+    """A small batch runs both local steps in one launch until the caller sets
+    their shapes: then each is a launch of its own, one more per iteration."""
+    mesh = strip(12, 12)
+    cfg = api.drape_config(max_iterations=6)
+    solvers = [api.ProjectiveDynamicsSolver().init_explicit(mesh, cfg, api.SetupDesc(), pinned=mesh.pinned) for _ in range(2)]
+    batch = api.Batch(solvers)
+    batch.step(DT)
+    launches, want = batch.launches_per_step(), batch.state(0)[0]
+    for shape in ((1, 1), (2, 2), (1, 2), (2, 1)):
+        batch.set_local_shape(*shape)
+        for k in range(2):
+            batch.set_state(k, np.stack([mesh.px, mesh.py, mesh.pz], 1))
+        batch.step(DT)
+        assert batch.launches_per_step() == launches + 6, shape
+        assert np.array_equal(batch.state(0)[0], want), shape

@@ -486,7 +486,8 @@ class Batch:
         return v.value
 
     def set_local_shape(self, triangles_per_thread: int, hinges_per_thread: int):
-        """Elements per thread of the membrane and bending steps (1 or 2 each)."""
+        """Elements per thread of the membrane and bending steps (1 or 2 each),
+        each step a launch of its own."""
         L.check(L.lib().vistio_batch_set_local_shape(self.h, int(triangles_per_thread), int(hinges_per_thread)),
                 self.ctx.h)
 

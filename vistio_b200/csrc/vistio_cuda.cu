@@ -168,6 +168,7 @@ struct vistio_batch {
   std::vector<uint64_t> sn_key;
   uint32_t warp_limit = kWarpItemLimit;             // s (s + m) limit of the warp items that share a unit
   uint32_t tri_per = 2, hinge_per = 1;              // elements per thread of k_tri / k_hinge (autotuned)
+  bool local_split = false;                         // a small batch too runs a kernel per local step, in these shapes
   uint32_t self_ccd_dedup = 1;                      // self CCD over each vertex-triangle test once
   float tuned_ms = 0.f;                             // sweep time of the tuned schedule (0: not tuned)
   float occ_ms[3] = {-1.f, -1.f, -1.f};  // the autotuner's times of the three forms (ms per solve)
@@ -1203,7 +1204,7 @@ uint32_t launch_solve(vistio_batch* b, cudaStream_t st, After after, uint32_t re
   return n;
 }
 
-// The local steps in the shapes the autotuner chose (elements per thread).
+// The local steps in the batch's shapes (elements per thread).
 void launch_membrane(vistio_batch* b, cudaStream_t st) {
   if (!b->n_tri_chunks) return;
   if (b->tri_per == 2) launch_pdl(k_tri, b->n_tri_chunks, kTriThreads, 0, st, b->dev);
@@ -1218,14 +1219,21 @@ void launch_bending(vistio_batch* b, cudaStream_t st) {
 // Element chunks (256 elements) of a batch whose local steps share one launch
 // (k_local). Whole plain steps of 10 iterations, two launches against one: 97x97
 // sheet (184 chunks) 517 -> 486 us, 24 sheets (1,620) 1860 -> 1840, 64 sheets
-// (7,700) 2508 -> 2544, 512 sheets 13.94 -> 14.60 ms.
+// (7,700) 2508 -> 2544, 512 sheets 13.94 -> 14.60 ms. A caller that sets the
+// shapes gets them, a launch each, and vistio_batch_tune_local times both ways.
 constexpr uint32_t kLocalChunks = 4 * 4 * 148;
+bool local_in_one(const vistio_batch* b) {
+  return b->n_tri_chunks && b->n_hinge_chunks && b->n_tri_chunks + b->n_hinge_chunks <= kLocalChunks;
+}
+void launch_local(vistio_batch* b, cudaStream_t st) {
+  launch_pdl(k_local, b->n_tri_chunks + b->n_hinge_chunks, kElemThreads, 0, st, b->dev, b->n_tri_chunks);
+}
 
 // One PD iteration up to and with the pass over the vertices after its solve.
 uint32_t launch_iteration(vistio_batch* b, cudaStream_t st, bool ipc, uint32_t refine) {
   uint32_t n = 1;
-  if (b->n_tri_chunks && b->n_hinge_chunks && b->n_tri_chunks + b->n_hinge_chunks <= kLocalChunks) {
-    launch_pdl(k_local, b->n_tri_chunks + b->n_hinge_chunks, kElemThreads, 0, st, b->dev, b->n_tri_chunks);
+  if (local_in_one(b) && !b->local_split) {
+    launch_local(b, st);
     ++n;
   } else {
     if (b->n_tri_chunks) { launch_membrane(b, st); ++n; }
@@ -2018,13 +2026,13 @@ vistio_status vistio_batch_tune_local(vistio_batch* b, uint32_t* tri_per_thread,
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  float ms[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c = 0; c < 4; ++c) {
+  float ms[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // membrane 1, 2, bending 1, 2, both in one launch
+  for (int c = 0; c < (local_in_one(b) ? 5 : 4); ++c) {
     const uint32_t per = 1u + uint32_t(c & 1);
-    if (c < 2) b->tri_per = per; else b->hinge_per = per;
+    if (c < 2) b->tri_per = per; else if (c < 4) b->hinge_per = per;
     for (int r = 0; r < 6; ++r) {  // one warm-up, five timed
       if (r == 1) CU(cudaEventRecord(e0, st));
-      if (c < 2) launch_membrane(b, st); else launch_bending(b, st);
+      if (c < 2) launch_membrane(b, st); else if (c < 4) launch_bending(b, st); else launch_local(b, st);
     }
     CU(cudaEventRecord(e1, st));
     CU(cudaEventSynchronize(e1));
@@ -2036,9 +2044,10 @@ vistio_status vistio_batch_tune_local(vistio_batch* b, uint32_t* tri_per_thread,
   CU(cudaGetLastError());
   b->tri_per = ms[1] <= ms[0] ? 2u : 1u;
   b->hinge_per = ms[3] < ms[2] ? 2u : 1u;
+  b->local_split = ms[4] > std::min(ms[0], ms[1]) + std::min(ms[2], ms[3]);
   if (tri_per_thread) *tri_per_thread = b->tri_per;
   if (hinge_per_thread) *hinge_per_thread = b->hinge_per;
-  if (candidate_ms) std::memcpy(candidate_ms, ms, sizeof(ms));
+  if (candidate_ms) std::memcpy(candidate_ms, ms, 4 * sizeof(float));
   return drop_graphs(b);
 }
 
@@ -2048,6 +2057,7 @@ vistio_status vistio_batch_set_local_shape(vistio_batch* b, uint32_t tri_per_thr
     return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "elements per thread must be 1 or 2");
   b->tri_per = tri_per_thread;
   b->hinge_per = hinge_per_thread;
+  b->local_split = true;
   return drop_graphs(b);
 }
 
