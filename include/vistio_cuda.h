@@ -278,7 +278,9 @@ vistio_status vistio_batch_info(const vistio_batch* b, uint32_t* n_instances, ui
  * chosen by timing this batch's forward and backward sweeps:
  * - the sweep kind: 0 = one kernel launch per level of the supernodal trees;
  *   1 = one dependency-driven launch for both directions, in which each
- *   supernode waits only for its own children (forward) or parent (backward);
+ *   supernode waits only for its own children (forward) or parent (backward),
+ *   or, for a batch whose factor is at most 128 MiB, connected parts of the trees
+ *   that a block sweeps by itself, a launch per phase of them;
  *   2 (batches with garment groups: at least 8 garments of one mesh topology)
  *   = the bottom of the groups' trees swept one lane per garment, before and
  *   after kind 1 sweeps the rest;
@@ -295,7 +297,8 @@ vistio_status vistio_batch_info(const vistio_batch* b, uint32_t* n_instances, ui
  * that warp-item limit). The fastest candidate is kept (*chosen_limit; the
  * kind from vistio_batch_get_sweep_mode, the group limit from
  * vistio_batch_get_group_limit). Without tuning: kind 2 if the batch has
- * garment groups, else kind 1, with the limits 6144. For kinds 1 and 2 the
+ * garment groups, else kind 1, with the limits 6144; until the kind is tuned or
+ * set, a factor of at most 128 MiB is swept as kind 1 either way. For kinds 1 and 2 the
  * chosen schedule is then timed with both compiled forms of the dependency-
  * driven kernel (vistio_batch_get_sweep_blocks). Captured step graphs are
  * rebuilt on the next step. Synchronises the batch's stream. */
@@ -336,7 +339,8 @@ vistio_status vistio_batch_set_warp_limit(vistio_batch* b, uint32_t limit);
 vistio_status vistio_batch_set_sweep_mode(vistio_batch* b, uint32_t mode);
 /* The sweep kind and warp-item limit in use. */
 vistio_status vistio_batch_get_sweep_mode(const vistio_batch* b, uint32_t* mode, uint32_t* warp_limit);
-/* The dependency-driven sweep kernel (kinds 1 and 2) is compiled in three
+/* The dependency-driven sweep kernel (kinds 1 and 2, but for factors of at most
+ * 128 MiB in kind 1, see vistio_batch_tune) is compiled in three
  * forms, named by resident blocks per SM: 5 and 4 (eight-warp blocks, 48 and
  * 64 registers per thread) and 2 (sixteen-warp blocks, whose units hold twice
  * as many items); no reference counterpart. vistio_batch_tune times the three

@@ -504,7 +504,8 @@ class Batch:
 
     def set_sweep_mode(self, mode: str):
         """"levels": one launch per level; "dataflow": one dependency-driven
-        launch for both directions; "grouped" (batches with garment groups:
+        launch for both directions (a factor of at most 128 MiB: a launch per
+        phase of connected parts of the trees); "grouped" (batches with garment groups:
         8 or more garments of one mesh topology): the groups' tree bottoms
         one lane per garment, the rest dependency-driven."""
         L.check(L.lib().vistio_batch_set_sweep_mode(self.h, self.SWEEP_MODES.index(mode)), self.ctx.h)

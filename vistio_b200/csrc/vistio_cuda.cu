@@ -8,12 +8,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/vistio_cuda.h"
@@ -21,6 +23,7 @@
 #include "factor_kernels.cuh"
 #include "self_contact.cuh"
 #include "setup.h"
+#include "unit_kernels.cuh"
 
 using namespace vistio;
 static_assert(kSubtreeFloats <= kWarpFloats, "a bottom subtree must fit one warp buffer");
@@ -176,9 +179,11 @@ struct vistio_batch {
   // (sixteen warps, units of 2 kUnitItems items); the autotuner's choice
   uint32_t sweep_occ = 4;
   uint32_t unit_items = kUnitItems;  // items per subtree or warp-supernode unit of the schedule
-  // sweeps: 0 = one launch per level (k_level), 1 = dependency-driven (k_sweep),
+  // sweeps: 0 = one launch per level (k_level), 1 = dependency-driven (k_sweep, or
+  // where the factor is small k_units),
   // 2 = garment groups' tree bottoms by k_gsweep, the rest by k_sweep
   uint32_t sweep_mode = 1;
+  bool mode_set = false;  // by the caller or the tuner
   std::vector<uint2> units_host;                    // k_sweep work units in forward order
   uint32_t n_units = 0, n_units_fwd = 0;
   std::vector<uint2> units_fwd_host;                // k_sweep forward units: top supernodes deepest first
@@ -188,6 +193,12 @@ struct vistio_batch {
   DevBuf<uint32_t> df_items_fwd;
   DevBuf<uint2> df_units;
   DevBuf<uint32_t> df_parent, df_nkids, df_kid_ptr, df_kids, df_cnt, df_flag, df_queue;
+  // the units of a batch with a small factor (k_units), by phase
+  struct UnitPhase { uint32_t first, count, below, smem; };  // below: those without a root
+  std::vector<UnitPhase> unit_phases;
+  DevBuf<SweepUnitDev> units;
+  DevBuf<UnitNode> unit_nodes;
+  DevBuf<uint32_t> unit_tables;
   DevBuf<SnDev> sn;
   DevBuf<float4> U;
   // garment groups (k_gsweep, sweep mode 2): the bottom of the trees of
@@ -412,6 +423,321 @@ cudaError_t schedule_groups(vistio_batch* b, uint32_t limit, cudaStream_t st) {
 inline uint64_t pad4(uint64_t n) { return (n + 3) & ~3ull; }
 float estimate_kappa(const vistio_solver_config& c, const InstanceSetup& I);
 
+// The units of one symbolic structure (unit_kernels.cuh), with rows, places in U and
+// values counted from its garment's first, and the phase of each.
+struct UnitPlan {
+  std::vector<SweepUnitDev> units;
+  std::vector<uint32_t> phase, smem;
+  std::vector<UnitNode> nodes;
+  std::vector<uint32_t> table;
+};
+
+// Units sweep the batches whose factor is at most kUnitFactor bytes, about what L2
+// holds: above it a block's loads from HBM and its levels take turns. Plain steps of 10
+// iterations with their read-back, k_sweep against units: side 20 638 -> 390 us, 64
+// 1428 -> 722, 97 1819 -> 1056, 150 2916 -> 1501; 16 of 64 1666 -> 860, 64 of 64 (90 MB)
+// 2682 -> 2145, 16 of 128 (117 MB) 3728 -> 2698; but 64 of 97 (241 MB) 4581 -> 6162 and
+// 256 of 64 (362 MB) 5625 -> 7136.
+// A unit has up to kUnitBudget bytes, where the batch has more garments than
+// kWideMaxInstances kUnitBudgetMany: two blocks to an SM. 224 / 160 / 110 / 90 KB: side
+// 64 814 / 720 / 753 / 776 us, 97 1074 / 1063 / 1106 / 1056, 190 2318 / 2143 / 2345 /
+// 2131. 220 / 160 / 108 / 72 KB: 24 sheets of sides 17 to 151 3521 / 3603 / 2967 / 3439,
+// 16 of 97 2080 / 2093 / 1980 / 2013, 64 of 64 2615 / 2080 / 2198 / 2700.
+constexpr uint64_t kUnitFactor = 128ull << 20, kUnitBudget = 160 * 1024, kUnitBudgetMany = 108 * 1024;
+
+// Cuts a supernodal tree into units of about `budget` bytes of shared memory: first
+// every subtree that fits is a unit, then every subtree of what remains, and so on. A
+// supernode too large for shared memory is a unit whose values pass through it.
+// sn: the garment's supernodes. False if a unit does not fit after all.
+bool plan_units(const Factor& F, const SnDev* sn, uint64_t budget, UnitPlan& P) {
+  P = UnitPlan{};
+  const uint32_t n = uint32_t(F.sn.size()), none = UINT32_MAX;
+  auto tiles = [](uint32_t x) { return (x + 31) / 32; };
+  auto width = [](const Supernode& S) {
+    uint32_t w = 1;
+    while (w < S.ncols) w <<= 1;
+    return w;
+  };
+  auto in_warp = [](const Supernode& S) { return warp_item(S.ncols, S.nrows); };
+  auto diag_parts = [&](const Supernode& S) {
+    const uint32_t s = S.ncols, cw = unit_diag_cols(s);
+    return !in_warp(S) && unit_diag_split(s) ? (s + cw - 1) / cw * kTeam : 0u;
+  };
+  auto cost = [&](uint32_t k) {
+    const Supernode& S = F.sn[k];
+    return 4 * sn_floats(S.ncols, S.nrows) + 56ull * (S.ncols + 4) + 28ull * (S.nrows + 4) + 160 +
+           (in_warp(S) ? 0 : 16ull * std::max(kTeam, diag_parts(S)));
+  };
+  std::vector<uint32_t> unit(n, none), now(n);
+  std::vector<uint64_t> rest(n);
+  uint32_t nunits = 0;
+  for (uint32_t left = n; left;) {
+    std::fill(rest.begin(), rest.end(), 0);
+    std::fill(now.begin(), now.end(), none);
+    for (uint32_t k = 0; k < n; ++k) {  // children precede parents
+      if (unit[k] != none) continue;
+      rest[k] += cost(k);
+      if (F.sn[k].parent != none) rest[F.sn[k].parent] += rest[k];
+    }
+    for (uint32_t k = n; k-- > 0;) {
+      if (unit[k] != none) continue;
+      const uint32_t p = F.sn[k].parent;
+      if (p != none && now[p] != none) now[k] = now[p];
+      else if (rest[k] <= budget || rest[k] == cost(k)) now[k] = nunits++;  // a leaf of what remains is a unit at least
+      left -= now[k] != none;
+    }
+    for (uint32_t k = 0; k < n; ++k)
+      if (now[k] != none) unit[k] = now[k];
+  }
+  std::vector<std::vector<uint32_t>> members(nunits);
+  P.phase.assign(nunits, 0);
+  for (uint32_t k = 0; k < n; ++k) {
+    members[unit[k]].push_back(k);
+    const uint32_t p = F.sn[k].parent;
+    if (p != none && unit[p] != unit[k]) P.phase[unit[p]] = std::max(P.phase[unit[p]], P.phase[unit[k]] + 1);
+  }
+  // per row its unit, and its place in the z of the unit at hand
+  std::vector<uint32_t> unit_of(F.n), z_of(F.n, none);
+  for (uint32_t k = 0; k < n; ++k)
+    std::fill(unit_of.begin() + F.sn[k].first, unit_of.begin() + F.sn[k].first + F.sn[k].ncols, unit[k]);
+  // per panel row its entry in the pull lists, then for rows of its unit its kept update
+  std::vector<uint32_t> level(n, 0), place(F.fwd_sn.size());
+  for (uint32_t q = 0; q < F.fwd_sn.size(); ++q) place[F.sn[F.fwd_sn[q]].rows_off + F.fwd_pos[q]] = q | kAbove;
+  P.nodes.reserve(n);
+  P.table.reserve(8 * F.n + 4 * F.rows.size());
+  std::vector<UnitLevel> levels;
+  std::vector<uint32_t> tasks, row_of, list0, nlist, val_ptr, slots, x_of, val_of;
+  for (uint32_t u = 0; u < nunits; ++u) {
+    const std::vector<uint32_t>& mem = members[u];
+    const uint32_t top = mem.back();
+    // levels within the unit; at most one split diagonal product each
+    std::vector<std::vector<uint32_t>> lvl;
+    std::vector<uint8_t> has_diag;
+    for (uint32_t k : mem) {
+      const uint32_t p = F.sn[k].parent;
+      const bool d = diag_parts(F.sn[k]) > 0;
+      while (d && level[k] < has_diag.size() && has_diag[level[k]]) ++level[k];
+      if (level[k] >= lvl.size()) { lvl.resize(level[k] + 1); has_diag.resize(level[k] + 1, 0); }
+      lvl[level[k]].push_back(k);
+      has_diag[level[k]] |= d;
+      if (p != none && unit[p] == u) level[p] = std::max(level[p], level[k] + 1);
+    }
+    for (auto* v : {&tasks, &row_of, &list0, &nlist, &val_ptr, &slots, &x_of, &val_of}) v->clear();
+    levels.clear();
+    SweepUnitDev U{};
+    U.node0 = uint32_t(P.nodes.size()); U.nnodes = uint32_t(mem.size()); U.nlevels = uint32_t(lvl.size());
+    U.root = F.sn[top].parent == none; U.nabove = F.sn[top].nrows;
+    const UnitNode* nodes = nullptr;
+    uint32_t floats = 0, nrows = 0, pmax = 0, xmax = 0, ldmax = 1;
+    for (const auto& list : lvl) {
+      UnitLevel L{};
+      uint32_t part0 = 0, x0 = 0;
+      const uint32_t id0 = uint32_t(P.nodes.size()) - U.node0;
+      for (uint32_t k : list) {
+        const Supernode& S = F.sn[k];
+        const uint32_t s = S.ncols, m = S.nrows, ld = sn_ld(s), p_rel = uint32_t(sn[k].p_off - sn[k].d_off);
+        UnitNode N{};
+        N.src = sn[k].d_off - sn[0].d_off;
+        N.p_rel = p_rel;
+        N.len = uint32_t(pad4(p_rel + uint64_t(m) * ld));
+        N.at = floats; floats += N.len;
+        N.s = s; N.m = m; N.row0 = S.first;
+        N.col0 = U.ncols; U.ncols += (s + 7) & ~7u;
+        N.r0 = nrows; nrows += m;
+        N.x0 = x0; x0 += (m + 7) & ~7u;
+        ldmax = std::max(ldmax, ld);
+        N.width = in_warp(S) ? 0u : width(S);
+        N.chunk = p_rel + m * ld + m + 8 <= kTeamFloats ? kTeam : std::max(1u, std::min((kTeamFloats - 8) / ld, kTeam));
+        if (N.width && N.width < kTeam) { N.part0 = part0; part0 += kTeam; L.flags |= UnitLevel::kSplit; }
+        if (s > 32) L.flags |= UnitLevel::kWide;
+        if (diag_parts(S)) L.diag = uint32_t(P.nodes.size()) - U.node0 + 1;
+        pmax = std::max({pmax, part0, diag_parts(S)});
+        // per column: the descendants' updates before the first one from inside the
+        // unit are subtracted when it starts, the others kept
+        for (uint32_t c = 0; c < s; ++c) {
+          z_of[S.first + c] = N.col0 + c;
+          row_of.push_back(S.first + c);
+          val_ptr.push_back(uint32_t(slots.size()));
+          const uint32_t q0 = F.fwd_ptr[S.first + c], qe = F.fwd_ptr[S.first + c + 1];
+          uint32_t q = q0;
+          while (q < qe && unit[F.fwd_sn[q]] != u) ++q;
+          list0.push_back(q0);
+          nlist.push_back(q - q0);
+          U.lists |= q > q0;
+          for (; q < qe; ++q) {
+            const uint32_t d = F.fwd_sn[q];
+            if (unit[d] == u) place[F.sn[d].rows_off + F.fwd_pos[q]] = uint32_t(slots.size());
+            slots.push_back(unit[d] == u ? kInside : q);
+          }
+        }
+        for (uint32_t c = s; c & 7u; ++c) {
+          row_of.push_back(kNoRow);
+          list0.push_back(0);
+          nlist.push_back(0);
+          val_ptr.push_back(uint32_t(slots.size()));
+        }
+        P.nodes.push_back(N);
+      }
+      xmax = std::max(xmax, x0);
+      const uint32_t id1 = uint32_t(P.nodes.size()) - U.node0;
+      nodes = P.nodes.data() + U.node0;
+      auto make = [&](uint32_t& first, uint32_t& count, auto of) {  // the tasks `of` gives of each node
+        first = uint32_t(tasks.size());
+        for (uint32_t q = id0; q < id1; ++q) of(q, nodes[q]);
+        count = uint32_t(tasks.size()) - first;
+      };
+      auto put = [&](uint32_t q, uint32_t len, uint32_t part) {
+        for (uint32_t t = 0; t < tiles(len); ++t) tasks.push_back(unit_task(q, t, part));
+      };
+      make(L.col_task, L.ncol, [&](uint32_t q, const UnitNode& N) { put(q, N.s, 0); });
+      make(L.push_task, L.npush, [&](uint32_t q, const UnitNode& N) { if (!unit_own_rows(N.s, N.m)) put(q, N.m, 0); });
+      make(L.x_task, L.nx, [&](uint32_t q, const UnitNode& N) { if (N.width) put(q, N.m, 0); });
+      make(L.sum_task, L.nsum, [&](uint32_t q, const UnitNode& N) {
+        for (uint32_t p = 0; p < (N.width ? kTeam / N.width : 1u); ++p) put(q, N.s, p);
+      });
+      levels.push_back(L);
+    }
+    val_ptr.push_back(uint32_t(slots.size()));
+    U.nvals = uint32_t(slots.size());
+    const uint32_t* above = F.rows.data() + F.sn[top].rows_off;  // every row above the unit
+    for (uint32_t i = 0; i < U.nabove; ++i) z_of[above[i]] = U.ncols + i;
+    uint32_t id = 0;
+    for (const auto& list : lvl)
+      for (uint32_t k : list) {
+        const uint32_t *R = F.rows.data() + F.sn[k].rows_off, *at = place.data() + F.sn[k].rows_off, m = nodes[id++].m;
+        for (uint32_t j = 0; j < m; ++j) {
+          const uint32_t z = z_of[R[j]];
+          if (z == none || (unit_of[R[j]] != u && (z < U.ncols || z - U.ncols >= U.nabove || above[z - U.ncols] != R[j]))) return false;  // no elimination tree
+          x_of.push_back(z);
+          val_of.push_back(at[j]);
+        }
+      }
+    for (uint32_t i = 0; i < U.nabove; ++i) z_of[above[i]] = none;
+    // the unit's table and shared memory
+    std::vector<uint32_t>& table = P.table;
+    U.table0 = uint32_t(table.size());
+    for (const UnitLevel& L : levels) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&L);
+      table.insert(table.end(), w, w + sizeof(UnitLevel) / 4);
+    }
+    auto put = [&](uint32_t& at, const uint32_t* v, size_t len) {
+      at = uint32_t(table.size()) - U.table0;
+      table.insert(table.end(), v, v + len);
+    };
+    auto put_all = [&](uint32_t& at, const std::vector<uint32_t>& v) { put(at, v.data(), v.size()); };
+    put_all(U.tasks, tasks); put_all(U.row_of, row_of); put_all(U.list0, list0); put_all(U.nlist, nlist);
+    put_all(U.val_ptr, val_ptr); put_all(U.slots, slots); put(U.above, above, U.nabove); put_all(U.x_of, x_of);
+    put_all(U.val_of, val_of);
+    table.resize((table.size() + 3) & ~size_t(3));
+    U.ntable = uint32_t(table.size()) - U.table0;
+    uint64_t o = 0;
+    auto room = [&](uint32_t& where, uint64_t bytes) { where = uint32_t(o); o += (bytes + 15) / 16; };
+    for (U.stream = 0; U.stream < 2; ++U.stream) {
+      uint32_t values = 0;
+      o = 0;
+      U.bytes = floats * 4;
+      room(values, U.stream ? 8ull * kStreamFloats : U.bytes + 4 * ((8 * ldmax + 3) & ~3ull));  // read beside the vectors' padding
+      room(U.nodes_at, U.nnodes * sizeof(UnitNode));
+      room(U.table_at, U.ntable * 4ull);
+      room(U.vals_at, U.nvals * 16ull);
+      room(U.z_at, (U.ncols + U.nabove) * 16ull);
+      room(U.t_at, U.ncols * 16ull);
+      room(U.x_at, U.stream ? 0 : xmax * 16ull);
+      room(U.part_at, std::max(pmax, U.stream ? kTeam : 0u) * 16ull);
+      if (o * 16 <= kUnitSmem || mem.size() > 1) break;
+    }
+    if (mem.size() > 4095 || o * 16 > kUnitSmem) return false;
+    P.units.push_back(U);
+    P.smem.push_back(uint32_t(o * 16));
+  }
+  return true;
+}
+
+// The units of a batch, planned once per symbolic structure (sclass: of each garment)
+// and uploaded phase by phase. No phases if some structure cannot be cut.
+cudaError_t schedule_units(vistio_batch* b, const std::vector<uint32_t>& sclass, cudaStream_t st) {
+  b->unit_phases.clear();
+  const uint32_t n = b->ninst;
+  std::vector<uint32_t> sn0(n), fwd0(n), leader;  // leader: a garment of each structure
+  uint64_t sns = 0, fwd = 0;
+  for (uint32_t g = 0; g < n; ++g) {
+    const Factor& F = b->solvers[g]->setup.factor;
+    sn0[g] = uint32_t(sns); fwd0[g] = uint32_t(fwd);
+    sns += F.sn.size(); fwd += F.fwd_sn.size();
+    if (sclass[g] >= leader.size()) leader.resize(sclass[g] + 1, UINT32_MAX);
+    if (leader[sclass[g]] == UINT32_MAX) leader[sclass[g]] = g;
+  }
+  if (fwd >= kAbove) return cudaSuccess;
+  std::vector<UnitPlan> plans(leader.size());
+  std::atomic<uint32_t> next{0};
+  std::atomic<bool> fit{true};
+  auto work = [&]() {
+    try {
+      for (uint32_t c; (c = next.fetch_add(1)) < leader.size() && fit;) {
+        bool ok = false;
+        for (uint64_t budget = n > kWideMaxInstances ? kUnitBudgetMany : kUnitBudget; !ok && budget > 8192; budget -= budget / 4)
+          ok = plan_units(b->solvers[leader[c]]->setup.factor, b->sn_host.data() + sn0[leader[c]], budget, plans[c]);
+        if (!ok) fit = false;
+      }
+    } catch (...) {  // out of host memory: the sweeps do without units
+      fit = false;
+    }
+  };
+  const uint32_t threads = std::min({uint32_t(leader.size()), std::max(1u, std::thread::hardware_concurrency()), 16u});
+  std::vector<std::thread> pool;
+  try {
+    for (uint32_t t = 1; t < threads; ++t) pool.emplace_back(work);
+  } catch (...) {  // no more threads to be had
+  }
+  work();
+  for (std::thread& t : pool) t.join();
+  if (!fit) return cudaSuccess;
+  std::vector<uint32_t> node0, table0;
+  uint64_t nnodes = 0, words = 0;
+  for (const UnitPlan& P : plans) {
+    node0.push_back(uint32_t(nnodes));
+    table0.push_back(uint32_t(words));
+    nnodes += P.nodes.size();
+    words += P.table.size();
+  }
+  if (words >= (1ull << 32)) return cudaSuccess;
+  // phase by phase; in each the units with a root last (they have no backward
+  // launch), else the heaviest first
+  struct Placed { uint32_t phase, smem; SweepUnitDev u; };
+  std::vector<Placed> all;
+  for (uint32_t g = 0; g < n; ++g) {
+    const uint32_t c = sclass[g];
+    for (size_t i = 0; i < plans[c].units.size(); ++i) {
+      SweepUnitDev U = plans[c].units[i];
+      U.node0 += node0[c]; U.table0 += table0[c];
+      U.inst = g; U.vals0 = b->sn_host[sn0[g]].d_off; U.vbase = b->sn_host[sn0[g]].vbase; U.u0 = fwd0[g];
+      all.push_back({plans[c].phase[i], plans[c].smem[i], U});
+    }
+  }
+  std::stable_sort(all.begin(), all.end(), [](const Placed& x, const Placed& y) {
+    return x.phase != y.phase ? x.phase < y.phase : x.u.root != y.u.root ? !x.u.root : x.u.bytes > y.u.bytes;
+  });
+  std::vector<SweepUnitDev> units;
+  for (const Placed& x : all) {
+    if (x.phase == b->unit_phases.size()) b->unit_phases.push_back({uint32_t(units.size()), 0, 0, 0});
+    vistio_batch::UnitPhase& P = b->unit_phases.back();
+    ++P.count;
+    P.below += !x.u.root;
+    P.smem = std::max(P.smem, x.smem);
+    units.push_back(x.u);
+  }
+  cudaError_t e = b->units.upload(units, st);
+  if (e == cudaSuccess) e = b->unit_nodes.alloc(nnodes, st);
+  if (e == cudaSuccess) e = b->unit_tables.alloc(words, st);
+  for (size_t c = 0; c < plans.size() && e == cudaSuccess; ++c) {
+    const UnitPlan& P = plans[c];
+    e = cudaMemcpyAsync(b->unit_nodes.p + node0[c], P.nodes.data(), P.nodes.size() * sizeof(UnitNode), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(b->unit_tables.p + table0[c], P.table.data(), P.table.size() * 4, cudaMemcpyHostToDevice, st);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  return e;
+}
+
 // Fronts of the device factorization are allocated for groups of garments
 // of at most this many bytes (at least one garment per group); one buffer
 // serves the groups one after another.
@@ -426,6 +752,8 @@ uint64_t instance_device_bytes(const InstanceSetup& I, bool refine, bool self_co
   const uint64_t V = I.nv, T = I.nt, H = I.nh, R = F.rows.size();
   uint64_t b = vals * 4 + F.sn.size() * sizeof(SnDev) + R * 4 + F.fwd_sn.size() * 4 + (V + 1) * 4 +
                F.sn.size() * 4 + R * 16;
+  if (vals * 4 <= kUnitFactor)  // the units of its sweeps: nodes, and the tables' words per task, column and row
+    b += F.sn.size() * (sizeof(UnitNode) + 4 * 4) + (V + 3 * F.sn.size()) * 5 * 4 + R * 3 * 4;
   b += V * (16 * 10 + 4 + 3 + 4 * 3) + T * (16 + 16 + 4 + 36 + 12) + H * (16 + 16 + 8 + 16 + 16) + (V + 1) * 8;
   if (refine || !F.numeric) b += (V + 1) * 4 + I.A_col.size() * 12;
   if (refine) b += V * 32;
@@ -1074,6 +1402,10 @@ vistio_status pack_batch(vistio_ctx* ctx, vistio_solver* const* solvers, uint32_
   }
   b->dev_w = d;
   b->dev_w.Y = b->W.p;
+  if (NVALS * 4 <= kUnitFactor) {
+    CU(schedule_units(b, gp.sclass, st));
+    b->device_bytes += b->units.n * sizeof(SweepUnitDev) + b->unit_nodes.n * sizeof(UnitNode) + b->unit_tables.n * 4;
+  }
   return VISTIO_OK;
 }
 
@@ -1159,6 +1491,18 @@ uint32_t launch_sweeps(vistio_batch* b, const BatchDev& dv, cudaStream_t st) {
       ++n;
     }
     if (gb) { launch_pdl(k_gsweep<1>, gb, kGThreads, kGSmem, st, dv, b->n_gitems_bwd); ++n; }
+    return n;
+  }
+  if (!b->unit_phases.empty() && (b->sweep_mode == 1 || (b->sweep_mode == 2 && !b->mode_set))) {
+    uint32_t n = 0;
+    auto launch = [&](auto kernel, const vistio_batch::UnitPhase& L, uint32_t count) {
+      if (!count) return;
+      launch_pdl(kernel, count, kUnitThreads, L.smem, st, dv, static_cast<const SweepUnitDev*>(b->units.p + L.first),
+                 static_cast<const UnitNode*>(b->unit_nodes.p), static_cast<const uint32_t*>(b->unit_tables.p));
+      ++n;
+    };
+    for (const auto& L : b->unit_phases) launch(k_units<0>, L, L.count);
+    for (size_t p = b->unit_phases.size(); p-- > 0;) launch(k_units<1>, b->unit_phases[p], b->unit_phases[p].below);
     return n;
   }
   if (b->sweep_mode == 1 && b->n_units) {
@@ -1475,6 +1819,8 @@ vistio_status vistio_ctx_create(int32_t device, vistio_ctx** out) {
   CU(cudaFuncSetAttribute(k_sweep<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   CU(cudaFuncSetAttribute(k_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   CU(cudaFuncSetAttribute(k_sweep<2, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
+  CU(cudaFuncSetAttribute(k_units<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUnitSmem));
+  CU(cudaFuncSetAttribute(k_units<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUnitSmem));
   CU(cudaFuncSetAttribute(k_gsweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
   CU(cudaFuncSetAttribute(k_gsweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
   {
@@ -1993,6 +2339,7 @@ vistio_status vistio_batch_tune(vistio_batch* b, uint32_t* chosen_limit, float* 
   CU(cudaStreamSynchronize(st));
   if (status & 4u) return fail(ctx, VISTIO_ERR_TIMEOUT, "a bounded wait of the sweeps gave up while tuning");
   b->tuned_ms = best;
+  b->mode_set = true;
   drop_graphs(b);
   if (chosen_limit) *chosen_limit = best_limit;
   return VISTIO_OK;
@@ -2085,6 +2432,7 @@ vistio_status vistio_batch_set_sweep_mode(vistio_batch* b, uint32_t mode) {
     return fail(b->ctx, VISTIO_ERR_INVALID_CONFIG, "sweep mode 2 needs garment groups (none in this batch)");
   vistio_ctx* ctx = b->ctx;
   b->sweep_mode = mode;
+  b->mode_set = true;
   std::vector<uint32_t> items = schedule_levels(b, b->warp_limit);  // mode 2 leaves the groups' supernodes out
   CU(upload_schedule(b, items, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
