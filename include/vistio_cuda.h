@@ -395,10 +395,11 @@ typedef struct vistio_server_config {
    * is overridden); 1: each request's own setting (0 = its cohort factorizes
    * on the GPU when it starts, on the thread that calls vistio_server_tick). */
   uint32_t gpu_factorization;
-  /* Sweep kind of every cohort (vistio_batch_set_sweep_mode): 0 = one launch
-   * per level, 1 = dependency-driven. Cohorts run side by side on their own
-   * streams, and the dependency-driven sweeps keep blocks resident that wait
-   * for one another, so 0 suits a busy server. */
+  /* Sweep kind of the cohorts whose factor is above 128 MiB
+   * (vistio_batch_set_sweep_mode): 0 = one launch per level, 1 = dependency-
+   * driven. Cohorts run side by side on their own streams, and those dependency-
+   * driven sweeps keep blocks resident that wait for one another, so 0 suits a
+   * busy server. Smaller factors are swept by units (vistio_batch_tune). */
   uint32_t sweep_mode;
   /* Admission window: while any cohort is running, ready requests of one step
    * configuration wait up to this long (from the first one's readiness) for

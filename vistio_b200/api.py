@@ -680,7 +680,8 @@ class Server:
                  gpu_factorization: bool = False, sweep_mode: str = "levels", admit_wait_ms: int = 0):
         """gpu_factorization False: the set-up threads factorize on the host,
         beside the GPU's work; True: each request's own host_factorization.
-        sweep_mode: the sweep kind of every cohort (Batch.SWEEP_MODES).
+        sweep_mode: the sweep kind of the cohorts whose factor is above 128 MiB
+        (Batch.SWEEP_MODES); smaller ones are swept by units.
         admit_wait_ms: while cohorts run, how long ready requests of one step
         configuration may wait for others to form a larger cohort."""
         cfg = L.ServerConfig(device, int(hbm_budget_bytes), int(max_cohort), int(setup_threads), int(steps_per_slice),

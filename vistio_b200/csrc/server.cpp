@@ -322,7 +322,12 @@ vistio_status start_cohort(vistio_server* S, const std::vector<Request*>& take, 
   std::vector<vistio_solver*> sv;
   for (Request* r : take) sv.push_back(r->solver);
   st = vistio_batch_create(c.ctx, sv.data(), uint32_t(sv.size()), &c.batch);
-  if (st == VISTIO_OK) st = vistio_batch_set_sweep_mode(c.batch, S->cfg.sweep_mode);
+  // A small factor is swept by units, whose blocks never wait for one another's (16
+  // requests a second for 10 s: latency p50 3.99 s with a launch per level, 0.85 so).
+  uint64_t factor_bytes = 0;
+  if (st == VISTIO_OK) st = vistio_batch_info(c.batch, nullptr, nullptr, nullptr, nullptr, &factor_bytes, nullptr);
+  if (st == VISTIO_OK)
+    st = vistio_batch_set_sweep_mode(c.batch, factor_bytes <= (128ull << 20) ? 1u : S->cfg.sweep_mode);
   if (st != VISTIO_OK) {
     std::string err = vistio_last_error(c.ctx);
     vistio_ctx_destroy(c.ctx);
