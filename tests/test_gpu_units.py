@@ -78,3 +78,23 @@ def test_dense_matrix(n):
     b = rng.normal(size=n).astype(np.float32)
     want = np.linalg.solve(a.astype(np.float64), b.astype(np.float64))
     assert np.linalg.norm(s.solve(b) - want) <= 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("blocks,size", [(1, 1), (300, 1), (257, 7), (40, 33)])
+def test_matrix_of_independent_blocks(blocks, size):
+    """Whole trees that share a unit: tridiagonal blocks."""
+    n = blocks * size
+    i = np.arange(n)
+    left, right = i % size > 0, i % size < size - 1
+    rows = np.concatenate([i, i[left], i[right]])
+    cols = np.concatenate([i, i[left] - 1, i[right] + 1])
+    vals = np.concatenate([3.0 + (i % 5), np.full(left.sum() + right.sum(), -1.0)]).astype(np.float32)
+    order = np.lexsort((cols, rows))
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.uint32)
+    s = api.SparseSolver()
+    s.factorize(ptr, cols[order].astype(np.uint32), vals[order], n)
+    a = np.zeros((n, n))
+    a[rows, cols] = vals
+    b = np.random.default_rng(n).normal(size=n).astype(np.float32)
+    want = np.linalg.solve(a, b.astype(np.float64))
+    assert np.linalg.norm(s.solve(b) - want) <= 1e-6 * np.linalg.norm(want)

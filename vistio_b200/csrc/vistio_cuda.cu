@@ -479,11 +479,23 @@ bool plan_units(const Factor& F, const SnDev* sn, uint64_t budget, UnitPlan& P) 
       rest[k] += cost(k);
       if (F.sn[k].parent != none) rest[F.sn[k].parent] += rest[k];
     }
+    uint32_t forest = none;  // whole trees share a unit (a matrix of many small blocks)
+    uint64_t trees = 0;
     for (uint32_t k = n; k-- > 0;) {
       if (unit[k] != none) continue;
       const uint32_t p = F.sn[k].parent;
-      if (p != none && now[p] != none) now[k] = now[p];
-      else if (rest[k] <= budget || rest[k] == cost(k)) now[k] = nunits++;  // a leaf of what remains is a unit at least
+      if (p != none && now[p] != none) {
+        now[k] = now[p];
+      } else if (p == none && rest[k] <= budget) {
+        if (forest == none || trees + rest[k] > budget) {
+          forest = nunits++;
+          trees = 0;
+        }
+        now[k] = forest;
+        trees += rest[k];
+      } else if (rest[k] <= budget || rest[k] == cost(k)) {  // a leaf of what remains is a unit at least
+        now[k] = nunits++;
+      }
       left -= now[k] != none;
     }
     for (uint32_t k = 0; k < n; ++k)
