@@ -436,7 +436,9 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_add(uint32_t* v, uint32_t n
 // alone with G = 1 / 4 / 8 4.77 / 4.11 / 4.08; with kWideLevels 7 and G = 4 / 8
 // 3.88 / 3.75, 8 and 8 3.70. A step of 64 drapes (795,264 triangles: the chip is
 // full, and it is bound by instructions at 10 of 32 threads) from the root 18.1 ms,
-// from the siblings with G = 1 / 2 / 4 17.5 / 17.8 / 18.3.
+// from the siblings with G = 1 / 2 / 4 17.5 / 17.8 / 18.3. Where the line lies, contact
+// steps of drapes with G = 1 / 8: 8,192 triangles 855 / 735 us, 37,636 1336 / 1214,
+// 65,536 1707 / 1723, 98,304 1905 / 1981, 262,144 3299 / 3616.
 constexpr uint32_t kPairBuf = 24;
 constexpr uint64_t kSharedLeaves = 148 * 2048 / 4;  // two rounds of eight threads per leaf
 template <uint32_t G> __global__ void __launch_bounds__(256) k_self_pairs(BatchDev B, SelfContactView S) {
